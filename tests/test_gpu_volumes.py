@@ -1,0 +1,35 @@
+"""3D ray operators at the ends of what they accept: a volume one voxel thick
+with more than 2^24 bricks, and volumes that cover part of the image."""
+import numpy as np
+import pytest
+
+from tval3g import capi
+from tval3g import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _geometry(p0, p1, rv):
+    E, R = len(p0), len(p1)
+    g = dict(numMPs=1, numPaths=E * R, E=E, R=R, use_path=np.arange(1, E * R + 1), rv_x=rv[2], rv_y=rv[1], rv_z=rv[0],
+             scale=1.0, xe=p0[:, 0], ye=p0[:, 1], ze=p0[:, 2], xr=p1[:, 0], yr=p1[:, 1], zr=p1[:, 2])
+    i, j = np.divmod(np.arange(E * R), R)
+    return g, W.bresenham_csr_3d(p0[i], p1[j], rv[2], rv[1])
+
+
+def test_adjoint_more_than_2_24_bricks(torch_cuda):
+    """1 x 32767 x 32767 voxels are 2^25 bricks; the rays lie in those from 2^24 on and below."""
+    torch = torch_cuda
+    rv = (32767, 32767, 1)
+    p0 = np.array([[0, 5, 32760], [0, 32766, 16390]])
+    p1 = np.array([[0, 32766, 32766], [0, 0, 0], [0, 32000, 32766]])
+    g, (off, pix) = _geometry(p0, p1, rv)
+    y = np.arange(1, 7, dtype=np.float32)   # whole numbers: every sum is exact
+    op = capi.Operator(capi.ray3d_problem(rv, g))
+    out = torch.full((op.cols,), 7.0, device="cuda")
+    op.apply(torch.tensor(y, device="cuda"), out, trans=True)
+    at, inv = np.unique(np.asarray(pix, np.int64), return_inverse=True)
+    want = np.bincount(inv, np.repeat(y, np.diff(off)))
+    assert np.array_equal(out[torch.tensor(at, device="cuda")].cpu().numpy(), want.astype(np.float32))
+    assert int(torch.count_nonzero(out)) == len(at)
+    op.close()

@@ -207,7 +207,8 @@ struct OpDev {
 	// A tile's words may be cut into parts, each with the stretch of the list
 	// that its words refer to (positions count from there): block b of a launch,
 	// b < tfull, takes the part vtile[b] = (tile | parts - 1 << 24 | part << 28,
-	// list offset in tmeas, list length, id), longest work first; word v of lane
+	// list offset in tmeas, list length, id), longest work first (tpart NULL: no
+	// tile is cut, and the first is the tile alone); word v of lane
 	// l of its pixel-warp w is sidx[woff[RAYT_WARPS id + w] + 32 v + l].  Parts of
 	// one tile leave FP64 sums in tpart (from slot tpoff[b] on) and count in
 	// tticket[tile].  The remaining blocks zero the tiles tempty that no ray

@@ -1284,6 +1284,7 @@ constexpr int RAYT_LIST_CHUNK = 8192;                    // list entries per bul
 // 10.6 17.1 18.8 16.4.  Of (256, 512), 256 tiles: whole 26.0, 8192 rays 25.6
 // with the index in L2 but 5 % slower with it from HBM.
 constexpr int TILE_PART = 6144, TILE_CUT = 148;
+static_assert(TILE_CUT < 1 << 24, "tile numbers beside part numbers (OpDev::vtile)");
 constexpr int TILE_PARTS = 16;                           // parts per tile at most
 constexpr int RAYT_ZERO_TILES = 16;                      // tiles without rays zeroed per block
 
@@ -1355,7 +1356,7 @@ __global__ void __launch_bounds__(RAYT_ADJ_THREADS, 2) k_ray_adj_tiled(const Ins
 		RAY_WAIT();
 		// tiles that no ray crosses (the launch order ends with them): zeros,
 		// RAYT_ZERO_TILES tiles per block, none of the list machinery
-		// (32-bit indices: tile counts stay below 2^24, and 64-bit ones here
+		// (32-bit indices: tile counts stay below 2^31, and 64-bit ones here
 		// cost the whole kernel eight registers)
 		const int e0 = op.tfull + (local - op.tfull) * RAYT_ZERO_TILES;
 		const int e1 = min(e0 + RAYT_ZERO_TILES, op.tcount);
@@ -1373,7 +1374,8 @@ __global__ void __launch_bounds__(RAYT_ADJ_THREADS, 2) k_ray_adj_tiled(const Ins
 		return;
 	}
 	const int4 vt = __ldg(op.vtile + local);
-	const int t = vt.x & 0xffffff, parts = (vt.x >> 24 & 15) + 1, part = (int)((unsigned)vt.x >> 28);
+	const bool cut = op.tpart != nullptr;   // else vt.x is the tile whole: volumes have up to 2^25 bricks
+	const int t = cut ? vt.x & 0xffffff : vt.x, parts = cut ? (vt.x >> 24 & 15) + 1 : 1, part = cut ? (int)((unsigned)vt.x >> 28) : 0;
 	const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	const unsigned bar_list = smem_u32(smem);
 	int *sb = reinterpret_cast<int *>(smem + 8);   // the pixel-warps' first words
@@ -1696,10 +1698,12 @@ static void upload_tiles(cudaStream_t s, std::vector<VTile> &vt, const std::vect
 	std::vector<int> first((size_t)nt, -1), poff(vt.size() + 1, 0);
 	std::vector<int4> h(vt.size() + 1);
 	int slots = 0, tmax = 0;
+	bool cut = false;
+	for (const VTile &v : vt) cut |= v.parts > 1;
 	for (size_t i = 0; i < vt.size(); i++) {
 		const VTile &v = vt[i];
-		h[i] = make_int4((int)((unsigned)v.tile | (unsigned)(v.parts - 1) << 24 | (unsigned)v.part << 28), v.list, v.len,
-		                 (int)v.id);
+		h[i] = make_int4(cut ? (int)((unsigned)v.tile | (unsigned)(v.parts - 1) << 24 | (unsigned)v.part << 28) : v.tile, v.list,
+		                 v.len, (int)v.id);
 		if (v.parts > 1 && first[v.tile] < 0) {
 			first[v.tile] = slots;
 			slots += v.parts;
