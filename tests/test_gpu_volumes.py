@@ -33,3 +33,23 @@ def test_adjoint_more_than_2_24_bricks(torch_cuda):
     assert np.array_equal(out[torch.tensor(at, device="cuda")].cpu().numpy(), want.astype(np.float32))
     assert int(torch.count_nonzero(out)) == len(at)
     op.close()
+
+
+@pytest.mark.parametrize("shape,rv", [((5, 5, 5), (5, 4, 4)), ((7, 9, 10), (5, 11, 11)), ((3, 40, 41), (5, 31, 31)),
+                                      ((13, 13, 13), (1, 40, 54))])
+def test_adjoint_of_a_volume_smaller_than_the_image(shape, rv, torch_cuda):
+    """Nothing is written past the image, although the last layer of bricks reaches beyond it."""
+    torch = torch_cuda
+    rng = np.random.default_rng(sum(shape))
+    n, guard = int(np.prod(shape)), 8192
+    assert n > np.prod(rv)
+    p0, p1 = (np.stack([rng.integers(0, s, k) for s in (rv[2], rv[1], rv[0])], 1) for k in (6, 9))
+    g, (off, pix) = _geometry(p0, p1, rv)
+    y = rng.integers(-9, 10, 54).astype(np.float32)
+    op = capi.Operator(capi.ray3d_problem(shape, g))
+    buf = torch.full((n + guard,), 7.0, device="cuda")
+    op.apply(torch.tensor(y, device="cuda"), buf[:n], trans=True)
+    out = buf.cpu().numpy()
+    assert np.array_equal(out[:np.prod(rv)], np.bincount(pix, np.repeat(y, np.diff(off)), np.prod(rv)).astype(np.float32))
+    assert np.all(out[n:] == 7.0)
+    op.close()

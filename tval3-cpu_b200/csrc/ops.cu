@@ -1338,8 +1338,9 @@ __device__ __forceinline__ void tiled_store(const Inst &I, const OpDev &op, VecS
 		const int x = (t % op.ntx) * BRICK_X + px % BRICK_X;
 		const int y = ((t % bxy) / op.ntx) * BRICK_Y + (px / BRICK_X) % BRICK_Y;
 		const int z = (t / bxy) * BRICK_Z + px / (BRICK_X * BRICK_Y);
-		if (x < op.rvx && y < op.rvy && (long long)z * op.rvx * op.rvy < I.n)
-			vselw(I, ys)[x + (long long)y * op.rvx + (long long)z * op.rvx * op.rvy] = v;
+		// (the last layer of bricks may reach beyond the image's end, where the volume is smaller than the image)
+		const long long p = x + (long long)y * op.rvx + (long long)z * op.rvx * op.rvy;
+		if (x < op.rvx && y < op.rvy && p < I.n) vselw(I, ys)[p] = v;
 		return;
 	}
 	const int x = (t % op.ntx) * RAYT + (px % RAYT), row = (t / op.ntx) * RAYT + (px / RAYT);
