@@ -38,7 +38,8 @@ def test_adjoint_more_than_2_24_bricks(torch_cuda):
 @pytest.mark.parametrize("shape,rv", [((5, 5, 5), (5, 4, 4)), ((7, 9, 10), (5, 11, 11)), ((3, 40, 41), (5, 31, 31)),
                                       ((13, 13, 13), (1, 40, 54))])
 def test_adjoint_of_a_volume_smaller_than_the_image(shape, rv, torch_cuda):
-    """Nothing is written past the image, although the last layer of bricks reaches beyond it."""
+    """Nothing is written past the image, although the last layer of bricks reaches beyond it; between the volume's end
+    and the image's lie zeros, in the adjoint and in the normal product."""
     torch = torch_cuda
     rng = np.random.default_rng(sum(shape))
     n, guard = int(np.prod(shape)), 8192
@@ -52,4 +53,12 @@ def test_adjoint_of_a_volume_smaller_than_the_image(shape, rv, torch_cuda):
     out = buf.cpu().numpy()
     assert np.array_equal(out[:np.prod(rv)], np.bincount(pix, np.repeat(y, np.diff(off)), np.prod(rv)).astype(np.float32))
     assert np.all(out[n:] == 7.0)
+    assert np.all(out[np.prod(rv):n] == 0)
+    x = torch.tensor(rng.integers(-9, 10, n).astype(np.float32), device="cuda")
+    Ax, want = torch.empty(54, device="cuda"), torch.full((n,), 7.0, device="cuda")
+    op.apply(x, Ax)
+    op.apply(Ax, want, trans=True)
+    buf.fill_(7.0)
+    op.apply(x, buf[:n], trans=2)
+    assert torch.equal(buf[:n], want) and torch.all(buf[n:] == 7.0)
     op.close()

@@ -30,6 +30,7 @@ struct tval3g_operator {
 	float *d_au = nullptr;    // A x of a normal product (trans = 2)
 	cudaStream_t s = nullptr;
 	long long rows = 0, cols = 0;
+	long long written = 0;    // elements of A^T x that the adjoint's kernels cover; the rest are zeros
 };
 
 #define CAPI_BEGIN try {
@@ -246,6 +247,8 @@ int tval3g_op_create(tval3g_operator **out, const tval3g_problem *prob, int flag
 		I.op = op->st.dev;
 		op->rows = I.m;
 		op->cols = I.n;
+		// bricks cover the geometry's volume, which may be smaller than the image
+		op->written = I.op.tiled && I.op.tile3 ? (long long)p.rv_x * p.rv_y * p.rv_z : I.n;
 		TG_CUDA(cudaMalloc(&op->d_ctrl, sizeof(Ctrl)));
 		TG_CUDA(cudaMemsetAsync(op->d_ctrl, 0, sizeof(Ctrl), op->s));
 		I.ctrl = op->d_ctrl;
@@ -327,6 +330,8 @@ int tval3g_op_apply_n(tval3g_operator *op, int trans, const float *d_x, float *d
 	const VecSel xn{false, 0, x}, xm{true, 0, x}, yn{false, 0, d_y}, ym{true, 0, d_y};
 	const bool rays = op->st.dev.kind == TVAL3G_OP_RAY2D || op->st.dev.kind == TVAL3G_OP_RAY3D;
 	LaunchCtx L{s, op->d_inst, nullptr};
+	if (trans && op->written < op->cols)
+		TG_CUDA(cudaMemsetAsync(d_y + op->written, 0, sizeof(float) * (size_t)(op->cols - op->written), s));
 	if (trans == 2) {   // y = A^T (A x)
 		const VecSel au{true, 0, op->d_au};
 		if (rays) TG_CUDA(cudaMemsetAsync(op->d_au, 0, sizeof(float) * op->rows, s));
