@@ -16,6 +16,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import subprocess
+import unittest
 from dataclasses import dataclass
 
 import numpy as np
@@ -344,6 +345,8 @@ def ref_project3d(g, x, trans=False):
         path = os.path.join(HERE, "_ref", "libref_proj_3d.so")
         if not os.path.exists(path):
             build(reference=True)
+        if not os.path.exists(path):   # a test that compares with it is skipped
+            raise unittest.SkipTest("the reference's sources are not here: oracle/_ref is not built")
         L = C.CDLL(path)
         ip, i = C.POINTER(C.c_int), C.c_int
         L.ref3d_project.argtypes = [i, i, i, i, i, ip, ip, ip, ip, ip, ip, ip, i, i, i, C.c_float,
