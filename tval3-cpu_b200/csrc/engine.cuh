@@ -94,6 +94,26 @@ __device__ __forceinline__ float tfabs(float x) { return fabsf(x); }
 __device__ __forceinline__ double tfabs(double x) { return fabs(x); }
 __device__ __forceinline__ float tfma(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double tfma(double a, double b, double c) { return fma(a, b, c); }
+// An element of a vector that an earlier kernel of the chain wrote: an ordinary
+// global load.  __ldg (ld.global.nc) is for data that nothing writes while the
+// kernel is resident, and a dependent launch is resident while the kernel
+// before it still writes; the wait does not make such a load valid, and the
+// compiler may move it above the wait.
+__device__ __forceinline__ float ld_vec(const float *p) {
+	float v;
+	asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+	return v;
+}
+__device__ __forceinline__ double ld_vec(const double *p) {
+	double v;
+	asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+	return v;
+}
+__device__ __forceinline__ float4 ld_vec(const float4 *p) {
+	float4 v;
+	asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+	return v;
+}
 // a - b, never fused with a product that b is
 __device__ __forceinline__ float tsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ double tsub(double a, double b) { return __dsub_rn(a, b); }

@@ -61,13 +61,13 @@ __device__ __forceinline__ double dense_row4(const float4 *__restrict__ a, const
 #pragma unroll
 		for (int u = 0; u < U; u++) {
 			av[u] = __ldg(a + j + u * STEP);
-			xv[u] = __ldg(x + j + u * STEP);
+			xv[u] = ld_vec(x + j + u * STEP);
 		}
 #pragma unroll
 		for (int u = 0; u < U; u++) add(av[u], xv[u]);
 	}
 #pragma unroll 2
-	for (; j < n4; j += STEP) add(__ldg(a + j), __ldg(x + j));
+	for (; j < n4; j += STEP) add(__ldg(a + j), ld_vec(x + j));
 	return acc;
 }
 
@@ -76,7 +76,7 @@ __device__ __forceinline__ double dense_row4(const float4 *__restrict__ a, const
 __device__ __forceinline__ double dense_row1d(const real *__restrict__ a, const real *__restrict__ x, int n, int sub) {
 	double acc = 0.0;
 #pragma unroll 4
-	for (int j = sub * 32 + (threadIdx.x & 31); j < n; j += 32 * DENSE_WPR) acc = fma((double)__ldg(a + j), (double)__ldg(x + j), acc);
+	for (int j = sub * 32 + (threadIdx.x & 31); j < n; j += 32 * DENSE_WPR) acc = fma((double)__ldg(a + j), (double)ld_vec(x + j), acc);
 	return acc;
 }
 
@@ -92,7 +92,7 @@ __device__ __forceinline__ double dense_row1(const real *__restrict__ a, const r
 #pragma unroll
 		for (int u = 0; u < CHUNK / 256; u++) {
 			const int j = c * CHUNK + u * 256 + threadIdx.x;
-			xv[u] = j < n ? __ldg(x + j) : (real)0;
+			xv[u] = j < n ? ld_vec(x + j) : (real)0;
 		}
 	};
 	double acc = 0.0;
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(256) k_dense_adj(const Inst *tab, TileMap map,
 				float4 av[4];
 #pragma unroll
 				for (int u = 0; u < 4; u++) {
-					xv[u] = __ldg(x + r + u);
+					xv[u] = ld_vec(x + r + u);
 					av[u] = __ldg(reinterpret_cast<const float4 *>(op.A + (r + u) * n + c0));
 				}
 #pragma unroll
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(256) k_dense_adj(const Inst *tab, TileMap map,
 				}
 			}
 			for (; r < r1; r++) {
-				real xv = __ldg(x + r);
+				real xv = ld_vec(x + r);
 				float4 av = __ldg(reinterpret_cast<const float4 *>(op.A + r * n + c0));
 				acc0 = fma((double)av.x, (double)xv, acc0);
 				acc1 = fma((double)av.y, (double)xv, acc1);
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(256) k_dense_adj(const Inst *tab, TileMap map,
 		}
 	} else {
 		for (long long r = r0; r < r1; r++) {
-			real xv = __ldg(x + r);
+			real xv = ld_vec(x + r);
 			const real *ar = op.A + r * n;
 			if (c0 + 0 < n) acc0 = fma((double)__ldg(ar + c0 + 0), (double)xv, acc0);
 			if (c0 + 1 < n) acc1 = fma((double)__ldg(ar + c0 + 1), (double)xv, acc1);
@@ -872,11 +872,11 @@ __global__ void __launch_bounds__(256) k_gather(const Inst *tab, TileMap map, in
 					vv[u] = __ldg(val + k + u * W);
 				}
 #pragma unroll
-				for (int u = 0; u < 4; u++) xx[u] = __ldg(x + ii[u]);
+				for (int u = 0; u < 4; u++) xx[u] = ld_vec(x + ii[u]);
 #pragma unroll
 				for (int u = 0; u < 4; u++) acc = fma((double)vv[u], (double)xx[u], acc);
 			}
-			for (; k < k1; k += W) acc = fma((double)__ldg(val + k), (double)__ldg(x + __ldg(ind + k)), acc);
+			for (; k < k1; k += W) acc = fma((double)__ldg(val + k), (double)ld_vec(x + __ldg(ind + k)), acc);
 		} else {
 			for (; k + 3 * W < k1; k += 4 * W) {
 				int ii[4];
@@ -884,11 +884,11 @@ __global__ void __launch_bounds__(256) k_gather(const Inst *tab, TileMap map, in
 #pragma unroll
 				for (int u = 0; u < 4; u++) ii[u] = __ldg(ind + k + u * W);
 #pragma unroll
-				for (int u = 0; u < 4; u++) xx[u] = __ldg(x + ii[u]);
+				for (int u = 0; u < 4; u++) xx[u] = ld_vec(x + ii[u]);
 #pragma unroll
 				for (int u = 0; u < 4; u++) acc += xx[u];
 			}
-			for (; k < k1; k += W) acc += __ldg(x + __ldg(ind + k));
+			for (; k < k1; k += W) acc += ld_vec(x + __ldg(ind + k));
 		}
 	}
 #pragma unroll
@@ -1023,14 +1023,14 @@ __global__ void __launch_bounds__(256) k_ray_fwd(const Inst *tab, TileMap map, i
 			real v[4];
 #pragma unroll
 			for (int u = 0; u < 4; u++) {
-				v[u] = __ldg(x + idx);
+				v[u] = ld_vec(x + idx);
 				step();
 			}
 			acc += (double)((v[0] + v[1]) + (v[2] + v[3]));
 		}
 		real rest = 0.f;
 		for (; j <= M; j += SUBW) {
-			rest += __ldg(x + idx);
+			rest += ld_vec(x + idx);
 			step();
 		}
 		acc += (double)rest;
@@ -1110,7 +1110,7 @@ __global__ void __launch_bounds__(RAY1_BLOCK) k_ray_fwd_thread(const Inst *tab, 
 		const real *p = x + (i1 + (D3 ? i2 * S2 : 0));
 		asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, %3;" : "+r"(f1), "+r"(i1) : "r"(df1), "r"(di1));
 		if (D3) asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, %3;" : "+r"(f2), "+r"(i2) : "r"(df2), "r"(di2));
-		return __ldg(p);
+		return ld_vec(p);
 	};
 	RAY_WAIT();
 	if (!x) x = vsel(I, xs);

@@ -176,11 +176,11 @@ __device__ __forceinline__ double row_sum(const Rows &R, long long row) {
 				vv[u] = R.val ? (double)__ldg(R.val + k + u * G) : R.w;
 			}
 #pragma unroll
-			for (int u = 0; u < 4; u++) xx[u] = __ldg(R.x + (long long)ii[u] * W + c);
+			for (int u = 0; u < 4; u++) xx[u] = ld_vec(R.x + (long long)ii[u] * W + c);
 #pragma unroll
 			for (int u = 0; u < 4; u++) acc += vv[u] * xx[u];
 		}
-		for (; k < k1; k += G) acc += (R.val ? (double)__ldg(R.val + k) : R.w) * __ldg(R.x + (long long)__ldg(R.ind + k) * W + c);
+		for (; k < k1; k += G) acc += (R.val ? (double)__ldg(R.val + k) : R.w) * ld_vec(R.x + (long long)__ldg(R.ind + k) * W + c);
 	}
 #pragma unroll
 	for (int o = 16; o >= W; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
