@@ -233,7 +233,10 @@ int tval3g_tune_stats(long long *measured, long long *cached);
  * (trans = 1) or the normal product y = A^T (A x) of the solve's get_g_mult
  * (trans = 2; a one-layer dense operator reads A once, as the reference's
  * cache-blocked dense path, 2d/tval3_cpu_2d.cpp:361-394) with DEVICE x, y
- * (lengths rows/cols as reported; both cols for trans = 2). */
+ * (lengths rows/cols as reported; both cols for trans = 2).  An operator keeps
+ * scratch for its products (partial sums, transposed images): products of one
+ * operator must not overlap on the device.  Enqueue them on one stream, or
+ * order the streams; one thread at a time, or an operator per thread. */
 typedef struct tval3g_operator tval3g_operator;
 int tval3g_op_create(tval3g_operator **op, const tval3g_problem *prob, int flags);
 int tval3g_op_shape(const tval3g_operator *op, long long *rows, long long *cols, long long *nnz);

@@ -242,7 +242,7 @@ struct OpDev {
 	int tmax;               // longest list of a block
 	const int4 *vtile;
 	const int *tmeas, *woff, *tempty, *tpoff;
-	int *tticket;
+	unsigned *tticket;
 	double *tpart;
 	const uint4 *sidx;
 	const unsigned char *tperm;

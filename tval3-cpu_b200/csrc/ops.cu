@@ -1483,8 +1483,9 @@ __global__ void __launch_bounds__(RAYT_ADJ_THREADS, 2) k_ray_adj_tiled(const Ins
 		__threadfence();
 		__syncthreads();
 		if (threadIdx.x == 0) {
-			last = atomicAdd(op.tticket + t, 1) == parts - 1;
-			if (last) op.tticket[t] = 0;
+			// (atomicInc wraps to 0 at parts - 1: also when two products overlapped
+			// against the rule, the count is back at 0 after both)
+			last = atomicInc(op.tticket + t, (unsigned)parts - 1u) == (unsigned)parts - 1u;
 		}
 		__syncthreads();
 		if (!last || threadIdx.x >= RAYT_THREADS) return;
@@ -1725,8 +1726,8 @@ static void upload_tiles(cudaStream_t s, std::vector<VTile> &vt, const std::vect
 	d.tticket = nullptr;
 	d.tpart = nullptr;
 	if (slots) {
-		d.tticket = (int *)up(nullptr, 0, sizeof(int) * (size_t)nt);
-		TG_CUDA(cudaMemsetAsync(d.tticket, 0, sizeof(int) * (size_t)nt, s));
+		d.tticket = (unsigned *)up(nullptr, 0, sizeof(unsigned) * (size_t)nt);
+		TG_CUDA(cudaMemsetAsync(d.tticket, 0, sizeof(unsigned) * (size_t)nt, s));
 		d.tpart = (double *)up(nullptr, 0, sizeof(double) * (size_t)slots * RAYT_THREADS);
 	}
 	d.tiled = 1;
