@@ -551,7 +551,9 @@ __global__ void __launch_bounds__(ROWS_THREADS, 1) k_dense_rows(const Inst *tab,
 	extern __shared__ __align__(128) unsigned char dsm[];
 	__shared__ unsigned long long full[ROWS_STAGES];
 	__shared__ double spart[2][R][ROWS_THREADS / 32];
-	__shared__ int s_abort;
+	// a wait gave up: one flag for each parity of the loop, so that a warp which
+	// is on to the next rows raises another flag than a slow one still reads
+	__shared__ int s_abort[2];
 	const OpDev &op = I.op;
 	const int m = (int)op.m, n = (int)op.n, n4 = n >> 2;
 	const int G = gridDim.x, c = blockIdx.x, rows = c < m ? (m - c + G - 1) / G : 0;
@@ -564,7 +566,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, 1) k_dense_rows(const Inst *tab,
 		bulk_g2s(smem_u32(dsm + (size_t)st * n * 4), A + (long long)(c + (long long)i * G) * n, 4u * n, bar0 + 8u * st);
 	};
 	if (threadIdx.x == 0) {
-		s_abort = 0;
+		s_abort[0] = s_abort[1] = 0;
 		for (int st = 0; st < stages; st++) mbar_init(bar0 + 8u * st, 1);
 		fence_mbar_init();
 		if (early)   // A is written by no kernel of the chain: the first rows before the wait
@@ -609,7 +611,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, 1) k_dense_rows(const Inst *tab,
 			w[r] = 0.0;
 			if (i + r >= rows) continue;
 			const bool ok = mbar_wait_warp(bar0 + 8u * st, (unsigned)((i + r) / stages) & 1u, err);
-			if (!ok && lane == 0) s_abort = 1;
+			if (!ok && lane == 0) s_abort[par] = 1;
 			if (!ok) continue;
 			if (EXACT) {   // short rows: converted once, products and sums in FP64
 #pragma unroll
@@ -649,7 +651,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, 1) k_dense_rows(const Inst *tab,
 		for (int r = 0; r < R; r++)
 			if (lane == r) spart[par][r][warp] = w[r];
 		__syncthreads();
-		if (s_abort) break;
+		if (s_abort[par]) break;
 		if (threadIdx.x == 0 && i > 0) {   // every thread has finished with the rows before: their stages may be refilled
 			fence_proxy_async_smem();
 			for (int r = i - R + stages; r < min(i + stages, rows); r++) issue(r);
