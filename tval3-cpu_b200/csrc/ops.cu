@@ -97,11 +97,12 @@ __device__ __forceinline__ double dense_row1(const real *__restrict__ a, const r
 	};
 	double acc = 0.0;
 	load_x(0);
-	for (int c = 0, buf = 0; c * CHUNK < n; c++, buf ^= 1) {
+	const int nc = (int)((n + (CHUNK - 1LL)) / CHUNK);   // (the last chunk's end may lie beyond the largest int)
+	for (int c = 0, buf = 0; c < nc; c++, buf ^= 1) {
 		double *bx = sx + buf * CHUNK;
 #pragma unroll
 		for (int u = 0; u < CHUNK / 256; u++) bx[u * 256 + threadIdx.x] = (double)xv[u];
-		if ((c + 1) * CHUNK < n) load_x(c + 1);
+		if (c + 1 < nc) load_x(c + 1);
 		const real *ac = a + (long long)c * CHUNK + first;
 		const int len = n - c * CHUNK;
 		if (len >= CHUNK) {
