@@ -201,8 +201,6 @@ struct OpDev {
 	// dense
 	const real *A;
 	int mrhs;              // layers on the tcgen05 3xTF32 path (mrhs.cu) instead of the gemv kernels
-	int dense_rows;        // rows per block of the forward product (1, 2, 4 or 8)
-	int dense_direct;      // 1: its rows straight from memory also where they are not float4 aligned
 	int dense_kchunks;     // row chunks of the transposed product
 	int fused_rpc;         // rows per CTA per band of the one-pass normal product (0: not used)
 	int fused_slab;        // its column slab per CTA

@@ -32,28 +32,41 @@ TG_BEGIN
 // ---------------------------------------------------------------------------
 // dense
 // ---------------------------------------------------------------------------
-// y = A x, every product formed and added in FP64.  A block's eight warps take
-// op.dense_rows rows, WARPS / dense_rows warps each:
-//   float4 aligned rows, and others of matrices up to DENSE_DIRECT elements:
-//     four warps a row, A and x straight from global memory.  What it needs is
-//     loads in flight: with one warp a row 4915 x 16384 took 115 us (four: 62;
-//     eight: 94), 1229 x 4096 11.7 (6.4), 691 x 2304 5.8 (4.8).
-//   unaligned rows of larger matrices, element by element: an eighth of the
-//     bytes per load, so x is converted once per block, chunk by chunk into
-//     shared memory, and a row takes one warp, or two to eight while the launch
-//     has fewer than DENSE_FWD_BLOCKS blocks: 4839 x 16129 79 us (85 with one
-//     warp and no shared memory, 103 with four), 3060 x 10201 35 (36, 45); at
-//     2167 x 7225 four warps straight from memory win, 14.9 to 15.8.
-constexpr int DENSE_WPR = 4;   // warps per float4 aligned row
-
-__device__ __forceinline__ double dense_row4(const float4 *__restrict__ a, const float4 *__restrict__ x, int n4, int sub) {
-	constexpr int STEP = 32 * DENSE_WPR, U = 4;
-	double acc = 0.0;
-	auto add = [&](const float4 &av, const float4 &xv) {
-		acc = fma((double)av.x, (double)xv.x, acc);
-		acc = fma((double)av.y, (double)xv.y, acc);
-		acc = fma((double)av.z, (double)xv.z, acc);
-		acc = fma((double)av.w, (double)xv.w, acc);
+// y = A x, every product formed and added in FP64, WPR warps per row (which of
+// the forms a launch takes: dense_form).  k_dense_fwd reads A and x straight
+// from global memory; k_dense_fwd_smem, for long rows that are not float4
+// aligned, has x converted once per block, chunk by chunk into shared memory.
+// The segments of 32 elements (float4s) that a row is read in go to CLASSES
+// classes in turn - four, fewer for long rows; lane l adds the l-th products of
+// a class in order, the lanes are added by halves, then the classes: the same
+// bits in a launch of few rows and of many.
+// Bound: the float-to-double conversions (two a product; with x in shared memory
+// one), A from memory where it is larger than L2; for few rows the loads in
+// flight.  Measured, us (one warp a row in one class, straight from memory -> this):
+//   few rows, aligned: 1229 x 4096 11.0 -> 5.8 (this with one warp a row 10.0),
+//   4915 x 16384 116 -> 57 (77); not aligned: 1116 x 3721 9.4 -> 5.1 (9.7), 1968 x
+//   6561 17.5 -> 10.9 (15.8), 3060 x 10201 35.8 -> 33 (34), 4839 x 16129 86 -> 66 (80)
+//   many rows: 8 layers of 1228 x 4096 24.0 -> 23.6 (this with four warps a row
+//   31), 16 of 188 x 625 5.3 -> 4.5 (8.1), of 1968 x 6561 103 -> 91 (two warps:
+//   116), of 4836 x 16129 832 -> 767 (824)
+//   FP64 build, an iteration of a solve: 1116 x 3721 33.0 with four warps, 34.6
+//   with one; 1968 x 6561 67.1 with four classes, 64.6 with one; 2764 x 9216 103
+//   and 100
+// acc += the row's products, by class (XA: x is float4 aligned too)
+template <int WPR, int CLASSES, bool XA>
+__device__ __forceinline__ void dense_row4(const float4 *__restrict__ a, const float *__restrict__ x, int n4, int sub,
+                                           double (&acc)[CLASSES / WPR]) {
+	constexpr int STEP = 32 * WPR, U = 4, NC = CLASSES / WPR;
+	auto load = [&](int j) {
+		if (XA) return ld_vec(reinterpret_cast<const float4 *>(x) + j);
+		const float *p = x + 4LL * j;
+		return make_float4(ld_vec(p), ld_vec(p + 1), ld_vec(p + 2), ld_vec(p + 3));
+	};
+	auto add = [&](double &s, const float4 &av, const float4 &xv) {
+		s = fma((double)av.x, (double)xv.x, s);
+		s = fma((double)av.y, (double)xv.y, s);
+		s = fma((double)av.z, (double)xv.z, s);
+		s = fma((double)av.w, (double)xv.w, s);
 	};
 	int j = sub * 32 + (threadIdx.x & 31);
 	for (; j + (U - 1) * STEP < n4; j += U * STEP) {   // U segments of the row in flight per lane
@@ -61,32 +74,51 @@ __device__ __forceinline__ double dense_row4(const float4 *__restrict__ a, const
 #pragma unroll
 		for (int u = 0; u < U; u++) {
 			av[u] = __ldg(a + j + u * STEP);
+			xv[u] = load(j + u * STEP);
+		}
+#pragma unroll
+		for (int u = 0; u < U; u++) add(acc[u % NC], av[u], xv[u]);
+	}
+#pragma unroll
+	for (int u = 0; u < U - 1; u++)
+		if (j + u * STEP < n4) add(acc[u % NC], __ldg(a + j + u * STEP), load(j + u * STEP));
+}
+
+// rows that are not float4 aligned and too short for shared memory (in the FP64
+// build: all): element by element, U in flight per lane
+template <int WPR, int CLASSES>
+__device__ __forceinline__ void dense_row1d(const real *__restrict__ a, const real *__restrict__ x, int n, int sub,
+                                            double (&acc)[CLASSES / WPR]) {
+	constexpr int STEP = 32 * WPR, U = 8, NC = CLASSES / WPR;
+	int j = sub * 32 + (threadIdx.x & 31);
+	for (; j + (U - 1) * STEP < n; j += U * STEP) {
+		real av[U], xv[U];
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			av[u] = __ldg(a + j + u * STEP);
 			xv[u] = ld_vec(x + j + u * STEP);
 		}
 #pragma unroll
-		for (int u = 0; u < U; u++) add(av[u], xv[u]);
+		for (int u = 0; u < U; u++) acc[u % NC] = fma((double)av[u], (double)xv[u], acc[u % NC]);
 	}
-#pragma unroll 2
-	for (; j < n4; j += STEP) add(__ldg(a + j), ld_vec(x + j));
-	return acc;
+#pragma unroll
+	for (int u = 0; u < U - 1; u++)
+		if (j + u * STEP < n) acc[u % NC] = fma((double)__ldg(a + j + u * STEP), (double)ld_vec(x + j + u * STEP), acc[u % NC]);
 }
 
-// rows that are not float4 aligned (or, in the FP64 build, doubles): element by
-// element, 32 warps-per-row apart
-__device__ __forceinline__ double dense_row1d(const real *__restrict__ a, const real *__restrict__ x, int n, int sub) {
-	double acc = 0.0;
-#pragma unroll 4
-	for (int j = sub * 32 + (threadIdx.x & 31); j < n; j += 32 * DENSE_WPR) acc = fma((double)__ldg(a + j), (double)ld_vec(x + j), acc);
-	return acc;
-}
-
-// the same with x in shared memory
-constexpr int DENSE_CHUNK = 2048;   // elements of x per chunk: 16 KB of doubles
-template <int WPR>
-__device__ __forceinline__ double dense_row1(const real *__restrict__ a, const real *__restrict__ x, int n, int sub,
-                                             double *sx) {
-	constexpr int STEP = 32 * WPR, CHUNK = DENSE_CHUNK, PER = CHUNK / STEP, G = PER < 8 ? PER : 8;   // (CHUNK doubles: one buffer)
-	const int lane = threadIdx.x & 31, first = sub * 32 + lane;
+#ifndef TVAL3G_FP64
+// the same with x in shared memory.  CLASSES 4: segment by segment in turn, as
+// above; 2: eight segments by eight, so that one warp a row adds each batch of
+// loads in one chain (segment by segment, three layers of 4836 x 16129 took 196
+// us instead of 167)
+template <int WPR, int CLASSES>
+__device__ __forceinline__ void dense_row1(const real *__restrict__ a, const real *__restrict__ x, int n, int sub,
+                                           double *sx, double (&acc)[CLASSES / WPR]) {
+	constexpr int CHUNK = DENSE_CHUNK, G = 8, GROUPS = CHUNK / (32 * WPR * G), NC = CLASSES / WPR;   // (CHUNK doubles: one buffer)
+	constexpr bool TURN = CLASSES == 4;
+	const int lane = threadIdx.x & 31;
+	auto at = [&](int g, int u) { return (TURN ? (g * G + u) * WPR + sub : (g * WPR + sub) * G + u) * 32 + lane; };
+	auto sum = [&](int g, int u) -> double & { return acc[(TURN ? u : g) % NC]; };
 	real xv[CHUNK / 256];
 	auto load_x = [&](int c) {
 #pragma unroll
@@ -95,7 +127,6 @@ __device__ __forceinline__ double dense_row1(const real *__restrict__ a, const r
 			xv[u] = j < n ? ld_vec(x + j) : (real)0;
 		}
 	};
-	double acc = 0.0;
 	load_x(0);
 	const int nc = (int)((n + (CHUNK - 1LL)) / CHUNK);   // (the last chunk's end may lie beyond the largest int)
 	for (int c = 0, buf = 0; c < nc; c++, buf ^= 1) {
@@ -103,67 +134,119 @@ __device__ __forceinline__ double dense_row1(const real *__restrict__ a, const r
 #pragma unroll
 		for (int u = 0; u < CHUNK / 256; u++) bx[u * 256 + threadIdx.x] = (double)xv[u];
 		if (c + 1 < nc) load_x(c + 1);
-		const real *ac = a + (long long)c * CHUNK + first;
+		const real *ac = a + (long long)c * CHUNK;
 		const int len = n - c * CHUNK;
 		if (len >= CHUNK) {
 			real av[2][G];
 #pragma unroll
-			for (int u = 0; u < G; u++) av[0][u] = __ldg(ac + u * STEP);
+			for (int u = 0; u < G; u++) av[0][u] = __ldg(ac + at(0, u));
 			__syncthreads();
 #pragma unroll
-			for (int g = 0; g < PER / G; g++) {
-				if (g + 1 < PER / G)
+			for (int g = 0; g < GROUPS; g++) {
+				if (g + 1 < GROUPS)
 #pragma unroll
-					for (int u = 0; u < G; u++) av[(g + 1) & 1][u] = __ldg(ac + ((g + 1) * G + u) * STEP);
+					for (int u = 0; u < G; u++) av[(g + 1) & 1][u] = __ldg(ac + at(g + 1, u));
 #pragma unroll
-				for (int u = 0; u < G; u++) acc = fma((double)av[g & 1][u], bx[first + (g * G + u) * STEP], acc);
+				for (int u = 0; u < G; u++) sum(g, u) = fma((double)av[g & 1][u], bx[at(g, u)], sum(g, u));
 			}
 		} else {
 			__syncthreads();
-#pragma unroll 4
-			for (int j = 0; first + j < len; j += STEP) acc = fma((double)__ldg(ac + j), bx[first + j], acc);
+			constexpr int GS = TURN ? 1 : NC;   // groups until the classes repeat
+			for (int g0 = 0; at(g0, 0) < len; g0 += GS)
+#pragma unroll
+				for (int g = 0; g < GS; g++)
+#pragma unroll
+					for (int u = 0; u < G; u++)
+						if (at(g0 + g, u) < len)
+							sum(g, u) = fma((double)__ldg(ac + at(g0 + g, u)), bx[at(g0 + g, u)], sum(g, u));
 		}
 	}
-	return acc;
 }
+#endif
 
+// the row of this thread's warp, one of WPR on it
+template <int WPR, int CLASSES>
+struct DenseRow {
+	static constexpr int NC = CLASSES / WPR;   // classes of a warp: sub, sub + WPR, ...
+	int n, sub;   // this warp: part sub of the row
+	unsigned row, layer;
+	const real *a, *x;   // (rows beyond the last: the last again, not stored)
+	double acc[NC] = {};
+	__device__ __forceinline__ DenseRow(const Inst &I, const VecSel &xs, int local) {
+		constexpr unsigned ROWS = WARPS / WPR;
+		const unsigned m = (unsigned)I.op.m, rt = (m + ROWS - 1) / ROWS, warp = threadIdx.x >> 5;
+		n = (int)I.op.n;
+		sub = (int)(warp % WPR);
+		layer = (unsigned)local / rt;
+		row = ((unsigned)local - layer * rt) * ROWS + warp / WPR;
+		a = I.op.A + (long long)min(row, m - 1) * n;
+		x = vsel(I, xs) + (long long)layer * n;
+	}
+	// y = the classes' sums over the lanes, added in order.  Class k's ends in
+	// lane k 32 / NC: at each level a lane gives away half of the classes that it
+	// still has (as warp_sums does).
+	__device__ __forceinline__ void store(const Inst &I, const VecSel &ys) {
+		const int lane = threadIdx.x & 31;
+#pragma unroll
+		for (int h = NC / 2, o = 16; h > 0; h >>= 1, o >>= 1) {
+			const bool up = lane & o;
+#pragma unroll
+			for (int k = 0; k < h; k++) {
+				const double give = up ? acc[k] : acc[k + h], keep = up ? acc[k + h] : acc[k];
+				acc[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+			}
+		}
+		double s = acc[0];
+#pragma unroll
+		for (int o = 16 / NC; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+		double t = 0.0;
+		if (WPR == 1) {
+			t = s;
+#pragma unroll
+			for (int k = 1; k < CLASSES; k++) t += __shfl_sync(0xffffffffu, s, k * (32 / NC));
+		} else {
+			__shared__ double ws[WARPS / WPR][CLASSES];
+			double *w = ws[(threadIdx.x >> 5) / WPR];
+			if (lane % (32 / NC) == 0) w[lane / (32 / NC) * WPR + sub] = s;
+			__syncthreads();
+			if (sub == 0 && lane == 0) {
+				t = w[0];
+#pragma unroll
+				for (int k = 1; k < CLASSES; k++) t += w[k];
+			}
+		}
+		if (sub == 0 && lane == 0 && row < I.op.m) vselw(I, ys)[layer * I.op.m + row] = (real)t;
+	}
+};
+
+template <int WPR, int CLASSES>
 __global__ void __launch_bounds__(256, 4) k_dense_fwd(const Inst *tab, TileMap map, int pred, VecSel xs, VecSel ys,
                                                       unsigned long long *launches) {
 	OPROLOGUE();
-	__shared__ double sx[2 * DENSE_CHUNK];
-	__shared__ double ws[WARPS];
-	const OpDev &op = I.op;
-	const long long m = op.m;
-	const int n = (int)op.n;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const int rows = op.dense_rows, wpr = WARPS / rows, sub = warp % wpr;   // this warp: part sub of its row
-	const long long rt = (m + rows - 1) / rows;
-	const long long layer = local / rt;
-	const long long row = (local - layer * rt) * rows + warp / wpr;
-	const real *x = vsel(I, xs) + layer * n;
-	const real *a = op.A + min(row, m - 1) * n;   // (rows beyond the last: the last again, not stored)
+	DenseRow<WPR, CLASSES> r(I, xs, local);
+#ifndef TVAL3G_FP64
 	// the same choice in every thread of the block
-	const bool vec = !FP64_BUILD && (n & 3) == 0 && ((reinterpret_cast<uintptr_t>(op.A) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
-	double acc;   // FP64 accumulation of the products
-	if (vec && wpr == DENSE_WPR)
-		acc = dense_row4(reinterpret_cast<const float4 *>(a), reinterpret_cast<const float4 *>(x), n >> 2, sub);
-	else if (op.dense_direct) acc = dense_row1d(a, x, n, sub);
-	else
-		switch (wpr) {
-		case 1: acc = dense_row1<1>(a, x, n, sub, sx); break;
-		case 2: acc = dense_row1<2>(a, x, n, sub, sx); break;
-		case 4: acc = dense_row1<4>(a, x, n, sub, sx); break;
-		default: acc = dense_row1<8>(a, x, n, sub, sx); break;
-		}
-	acc = warp_sum(acc);
-	if (wpr > 1) {
-		if (lane == 0) ws[warp] = acc;
-		__syncthreads();
-		if (sub == 0)
-			for (int w = 1; w < wpr; w++) acc += ws[warp + w];
-	}
-	if (sub == 0 && lane == 0 && row < m) vselw(I, ys)[layer * m + row] = (real)acc;
+	if ((r.n & 3) == 0 && (reinterpret_cast<uintptr_t>(I.op.A) & 15) == 0) {
+		const float4 *a4 = reinterpret_cast<const float4 *>(r.a);
+		if ((reinterpret_cast<uintptr_t>(r.x) & 15) == 0) dense_row4<WPR, CLASSES, true>(a4, r.x, r.n >> 2, r.sub, r.acc);
+		else dense_row4<WPR, CLASSES, false>(a4, r.x, r.n >> 2, r.sub, r.acc);
+	} else
+#endif
+		dense_row1d<WPR, CLASSES>(r.a, r.x, r.n, r.sub, r.acc);
+	r.store(I, ys);
 }
+
+#ifndef TVAL3G_FP64
+template <int WPR, int CLASSES>
+__global__ void __launch_bounds__(256, 4) k_dense_fwd_smem(const Inst *tab, TileMap map, int pred, VecSel xs, VecSel ys,
+                                                           unsigned long long *launches) {
+	OPROLOGUE();
+	__shared__ double sx[2 * DENSE_CHUNK];
+	DenseRow<WPR, CLASSES> r(I, xs, local);
+	dense_row1<WPR, CLASSES>(r.a, r.x, r.n, r.sub, sx, r.acc);
+	r.store(I, ys);
+}
+#endif
 
 // partial column sums of A^T x over one row chunk
 __global__ void __launch_bounds__(256) k_dense_adj(const Inst *tab, TileMap map, int pred, VecSel xs,
@@ -2093,10 +2176,19 @@ void op_forward(const LaunchCtx &L, const OpBatch &B, int pred, VecSel x, VecSel
 #ifndef TVAL3G_FP64
 	for (const auto &e : B.mrhs) mrhs_apply(L.stream, L.inst, e.first, pred, *e.second, false, x, y, ctr);
 #endif
-	const TileMap &df = unfused ? B.dense_fwd_nf : B.dense_fwd;
-	if (df.count > 0) {
-		launch_pdl(k_dense_fwd, df.count, 256, 0, L.stream, L.inst, df, pred, x, y, ctr);
-	}
+	const TileMap(&df)[DENSE_FORMS] = unfused ? B.dense_fwd_nf : B.dense_fwd;
+	auto dense = [&](auto kern, const TileMap &t) {
+		if (t.count > 0) launch_pdl(kern, t.count, 256, 0, L.stream, L.inst, t, pred, x, y, ctr);
+	};
+	dense(k_dense_fwd<1, 4>, df[DENSE_ONE]);
+	dense(k_dense_fwd<4, 4>, df[DENSE_FOUR]);
+#ifndef TVAL3G_FP64
+	dense(k_dense_fwd_smem<1, 4>, df[DENSE_SHORT]);
+	dense(k_dense_fwd_smem<1, 2>, df[DENSE_LONG_ONE]);
+	dense(k_dense_fwd_smem<2, 2>, df[DENSE_LONG_TWO]);
+#else
+	dense(k_dense_fwd<1, 1>, df[DENSE_LONG_ONE]);
+#endif
 	gather(L, B.csr_fwd, pred, 0, x, y);
 	if (B.ray2_transpose.count > 0 && !xT_ready) {
 		launch_pdl(k_transpose2d, B.ray2_transpose.count, 256, 0, L.stream, L.inst, B.ray2_transpose, pred, x, ctr);

@@ -11,8 +11,23 @@
 TG_BEGIN
 
 constexpr int WARPS = 8;   // warps per block in the operator kernels
-constexpr int DENSE_FWD_BLOCKS = 592;   // blocks that a dense forward launch with x in shared memory should have: four per SM
-constexpr long long DENSE_DIRECT = 16LL << 20;   // elements of a dense matrix whose unaligned rows are read without it
+// Forms of the dense forward: warps per row, x through shared memory or not.  In
+// a launch of few rows (all instances and layers counted) one warp a row leaves
+// too few loads in flight; in one of many, more warps a row only add prologues,
+// shuffles and barriers.  Rows that are not float4 aligned read x through shared
+// memory from two of its chunks on (LONG), for one warp a row from one (SHORT).
+// In the FP64 build nothing is converted and memory bounds long rows either way:
+// one warp, straight from memory.  Figures at k_dense_fwd.
+enum DenseForm { DENSE_ONE, DENSE_FOUR, DENSE_SHORT, DENSE_LONG_ONE, DENSE_LONG_TWO, DENSE_FORMS };
+constexpr int DENSE_CHUNK = 2048;   // elements of x per chunk: 16 KB of doubles
+inline DenseForm dense_form(long long rows, long long n, bool vec) {
+	const bool few = rows <= 1024 + n / 4;
+	if (!vec && n >= 2 * DENSE_CHUNK) return few && !FP64_BUILD ? DENSE_LONG_TWO : DENSE_LONG_ONE;
+	if (few) return DENSE_FOUR;
+	return !vec && n >= DENSE_CHUNK && !FP64_BUILD ? DENSE_SHORT : DENSE_ONE;
+}
+inline int dense_form_rows(DenseForm f) { return f == DENSE_FOUR ? 2 : f == DENSE_LONG_TWO ? 4 : 8; }   // per block
+
 // lanes per ray of the on-the-fly forward projectors where there are few rays
 // (below RAY1_MIN_RAYS): a warp traces 32 / RAY_SUBW rays at once, which spreads
 // the per-ray set-up (unpacking, the closed-form start of every lane, the final
@@ -33,7 +48,7 @@ constexpr long long RAY1_MIN_RAYS = 10240;
 struct OpBatch {
 	// dense (2d/mat_mult.h:15-36): forward gemv by rows; adjoint over
 	// (column tile, row chunk) blocks into partials, then a column reduction
-	TileMap dense_fwd, dense_adj, dense_red;
+	TileMap dense_fwd[DENSE_FORMS], dense_adj, dense_red;
 	real *dense_part = nullptr;
 	// dense operators whose normal product A^T (A u) reads A once: by rows
 	// (bands 0: k_dense_rows and k_dense_rows_red through dense_part) or, for wider
@@ -47,7 +62,7 @@ struct OpBatch {
 		int grid;        // CTAs of the by-rows form
 	};
 	std::vector<Fused> fused;
-	TileMap dense_fwd_nf, dense_adj_nf, dense_red_nf;
+	TileMap dense_fwd_nf[DENSE_FORMS], dense_adj_nf, dense_red_nf;
 	int fused_grid = 0;
 	long long fused_words = 0;   // band flags of all fused instances
 	int *fused_flags = nullptr;

@@ -522,20 +522,25 @@ static long long build_op_maps(std::vector<Inst> &inst, const std::vector<OpStor
 		ob.fused_words += bands;
 	}
 	// dense gemv maps: all dense instances, then those outside the fused set
-	for (int nf = 0; nf < 2; nf++) {
-		for (int i = 0; i < cnt; i++) {
-			OpDev &d = inst[i].op;
-			if (d.kind != TVAL3G_OP_DENSE || d.mrhs || (nf && d.fused_rpc)) continue;
-			const bool vec = !FP64_BUILD && d.n % 4 == 0 && (reinterpret_cast<uintptr_t>(d.A) & 15) == 0;
-			d.dense_direct = d.m * d.n <= DENSE_DIRECT;
-			d.dense_rows = WARPS;
-			if (vec || d.dense_direct) d.dense_rows = 2;   // four warps a row
-			else
-				while (d.dense_rows > 1 && d.layers * ((d.m + d.dense_rows - 1) / d.dense_rows) < DENSE_FWD_BLOCKS) d.dense_rows /= 2;
-			tb.add(i, d.layers * ((d.m + d.dense_rows - 1) / d.dense_rows));
+	// (fused instances: the launches of all, the others: the launches without them)
+	long long dense_rows[2] = {0, 0};
+	auto gemv = [&](const OpDev &d, int nf) { return d.kind == TVAL3G_OP_DENSE && !d.mrhs && !(nf && d.fused_rpc); };
+	for (int nf = 0; nf < 2; nf++)
+		for (int i = 0; i < cnt; i++)
+			if (gemv(inst[i].op, nf)) dense_rows[nf] += inst[i].op.layers * inst[i].op.m;
+	for (int nf = 0; nf < 2; nf++)
+		for (int f = 0; f < DENSE_FORMS; f++) {
+			for (int i = 0; i < cnt; i++) {
+				const OpDev &d = inst[i].op;
+				if (!gemv(d, nf)) continue;
+				const bool vec = !FP64_BUILD && d.n % 4 == 0 && (reinterpret_cast<uintptr_t>(d.A) & 15) == 0;
+				// (the same form, and so the same bits, in both maps)
+				if (dense_form(dense_rows[!d.fused_rpc], d.n, vec) != f) continue;
+				const int rows = dense_form_rows((DenseForm)f);
+				tb.add(i, d.layers * ((d.m + rows - 1) / rows));
+			}
+			tb.close(nf ? &ob.dense_fwd_nf[f] : &ob.dense_fwd[f]);
 		}
-		tb.close(nf ? &ob.dense_fwd_nf : &ob.dense_fwd);
-	}
 	for (int i = 0; i < cnt; i++) {
 		OpDev &d = inst[i].op;
 		if (d.kind != TVAL3G_OP_DENSE) continue;
