@@ -359,7 +359,8 @@ void prepare_op(cudaStream_t s, const tval3g_problem &p, int flags, OpStore &st,
 		d.scale = p.scale_factor;
 		d.rays = drays;
 		d.rays_fwd = drays;
-		if (is3 && nr >= RAY1_MIN_RAYS) {
+		const bool copies = is3 && nr >= RAY1_MIN_RAYS && !(flags & PLAN_LEAN);   // for the thread-per-ray form
+		if (copies) {
 			int4 *sorted = sort_rays_3d(s, (int)nr, drays, (long long)nmp * E);
 			st.owned.push_back(sorted);
 			st.bytes += (long long)sizeof(int4) * nr;
@@ -403,7 +404,7 @@ void prepare_op(cudaStream_t s, const tval3g_problem &p, int flags, OpStore &st,
 		}
 		// the image transposed (3D: every slice of the volume) for the forward
 		if (is3) {
-			if (d.nrays >= RAY1_MIN_RAYS) {   // only the thread-per-ray form reads it
+			if (copies) {
 				d.xT = dalloc_op<real>(s, st, (long long)p.rv_x * p.rv_y * p.rv_z);
 				d.tH = p.rv_y;
 				d.tslices = p.rv_z;
@@ -726,6 +727,17 @@ Plan::Plan(int count, const tval3g_problem *probs, const tval3g_options *opts, i
 	ops_.resize(count);
 	h_inst_.assign(count, Inst{});
 	try {
+		// vectors that would take more than FUSED_STEP_BYTES: one W and d (the
+		// iteration runs k_getg and k_shrink_grad), and 3D operators without the
+		// copies of the volume and the rays, so that the need stays the smaller one
+		long long all_n = 0;
+		for (int i = 0; i < count; i++) {
+			const tval3g_problem &p = probs[i];
+			any_cplx_ |= p.complex_data != 0;
+			all_n += ((long long)p.dim_x * p.dim_y * (p.dims == 3 ? p.dim_z : 1) * (p.complex_data ? 2 : 1) + 63) / 64 * 64;
+		}
+		const bool lean = NVN * all_n * (long long)sizeof(real) > FUSED_STEP_BYTES;
+		fused_step_ = !any_cplx_ && !lean;
 		// operators and sizes
 		for (int i = 0; i < count; i++) {
 			const tval3g_problem &p = probs[i];
@@ -733,7 +745,7 @@ Plan::Plan(int count, const tval3g_problem *probs, const tval3g_options *opts, i
 			                  : (p.op_kind == TVAL3G_OP_RAY3D) ? (long long)p.numPaths * p.numMPs
 			                  : (long long)p.m * (p.dims == 3 ? 1 : p.layers);
 			long long n = validate(p, b_len, 0, false);   // the callers validated p
-			prepare_op(stream_, p, flags, ops_[i], false);
+			prepare_op(stream_, p, flags | (lean ? PLAN_LEAN : 0), ops_[i], false);
 			Inst &I = h_inst_[i];
 			const int planes = p.complex_data ? 2 : 1;   // complex: real and imaginary planes
 			I.dims = p.dims; I.p = p.dim_y; I.q = p.dim_x; I.r = p.dims == 3 ? p.dim_z : planes;
@@ -755,7 +767,6 @@ Plan::Plan(int count, const tval3g_problem *probs, const tval3g_options *opts, i
 			I.numInit = o.numInitIterations;
 			I.skip_enabled = (o.skipMulRatio != 0 && p.op_kind != TVAL3G_OP_DENSE);
 			any_skip_ |= I.skip_enabled != 0;
-			any_cplx_ |= I.cplx != 0;
 #ifndef TVAL3G_FP64   // the autotuner measures the FP32 kernels
 			if (flags & TVAL3G_TUNE) autotune_operator(stream_, ops_[i], I);
 #endif
@@ -763,12 +774,8 @@ Plan::Plan(int count, const tval3g_problem *probs, const tval3g_options *opts, i
 		}
 		group_shared_dense(probs, flags);
 		// vectors: one arena, every vector 256-byte aligned
-		// (the second W and d last: complex plans do without, and plans whose
-		// vectors would take more than FUSED_STEP_BYTES, which keep the smaller
-		// need; their iteration runs k_getg and k_shrink_grad)
-		long long total = 0, all_n = 0;
-		for (const Inst &I : h_inst_) all_n += (I.n + 63) / 64 * 64;
-		fused_step_ = !any_cplx_ && NVN * all_n * (long long)sizeof(real) <= FUSED_STEP_BYTES;
+		// (the second W and d last)
+		long long total = 0;
 		const int nvn = fused_step_ ? NVN : vWx2;
 		std::vector<long long> base(count);
 		for (int i = 0; i < count; i++) {

@@ -46,6 +46,8 @@ long long build_op_maps_upload(std::vector<Inst> &inst, const std::vector<OpStor
 // internal plan flag: per-iteration (mu_k, beta_k) from set_schedule instead of
 // the continuation (every instance must have the same maxit)
 constexpr int PLAN_SCHEDULE = 1 << 16;
+// internal flag of prepare_op: without the copies that only make a 3D forward faster
+constexpr int PLAN_LEAN = 1 << 17;
 
 class Plan {
 public:
