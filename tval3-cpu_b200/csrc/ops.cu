@@ -1657,8 +1657,9 @@ __device__ __forceinline__ void part_words(int nv, int p, int parts, int &v0, in
 // pixel's positions ascend, so its first and last words' ends bound it; begun
 // on a 16-byte boundary) and, per part and warp of ranks, its word count (32 x
 // its share of the longest of the warp's lists, in 16-byte words).
-// parts[t TILE_PARTS + p] = (list offset in the tile, length, words, parts)
-__global__ void __launch_bounds__(RAYT_THREADS) k_tile_count(int ld, int H, int ntx, int nrays, int part,
+// parts[t stride + p] = (list offset in the tile, length, words, parts); stride:
+// TILE_PARTS, or 1 where no tile is cut
+__global__ void __launch_bounds__(RAYT_THREADS) k_tile_count(int ld, int H, int ntx, int nrays, int part, int stride,
                                                              const int *cptr, const int *cind, long long *tlen, long long *wlen,
                                                              int4 *parts, unsigned char *perm, unsigned *gbm) {
 	extern __shared__ unsigned bm[];   // nwords bits, then nwords exclusive prefix counts
@@ -1691,10 +1692,10 @@ __global__ void __launch_bounds__(RAYT_THREADS) k_tile_count(int ld, int H, int 
 	pixel[rank] = p;
 	__syncthreads();
 	const int nv = __reduce_max_sync(0xffffffffu, (byrank[threadIdx.x] + 7) >> 3);
-	const int np = max(1, min(min(TILE_PARTS, (int)(((long long)total + part - 1) / part)), (byrank[0] + 7) >> 3));
+	const int np = max(1, min(min(stride, (int)(((long long)total + part - 1) / part)), (byrank[0] + 7) >> 3));
 	p = pixel[threadIdx.x];
 	const int k0 = p >= 0 ? cptr[p] : 0, k1 = k0 + byrank[threadIdx.x];
-	for (int i = 0; i < TILE_PARTS; i++) {
+	for (int i = 0; i < stride; i++) {
 		int v0 = 0, v1 = 0;
 		if (i < np) part_words(nv, i, np, v0, v1);
 		const int ka = k0 + 8 * v0, kb = min(k1, k0 + 8 * v1);
@@ -1703,14 +1704,14 @@ __global__ void __launch_bounds__(RAYT_THREADS) k_tile_count(int ld, int H, int 
 			atomicMax(&hi[i], tile_pos(bm, pre, cind[kb - 1]));
 		}
 		if ((threadIdx.x & 31) == 0) {
-			wlen[((long long)t * TILE_PARTS + i) * RAYT_WARPS + (threadIdx.x >> 5)] = 32LL * (v1 - v0);
+			wlen[((long long)t * stride + i) * RAYT_WARPS + (threadIdx.x >> 5)] = 32LL * (v1 - v0);
 			atomicAdd(&wsum[i], v1 - v0);
 		}
 	}
 	__syncthreads();
-	if (threadIdx.x < TILE_PARTS) {
+	if (threadIdx.x < stride) {
 		const int i = threadIdx.x, a = hi[i] < 0 ? 0 : lo[i] & ~3;
-		parts[t * TILE_PARTS + i] = make_int4(a, hi[i] < 0 ? 0 : (hi[i] - a + 4) & ~3, wsum[i], np);
+		parts[(long long)t * stride + i] = make_int4(a, hi[i] < 0 ? 0 : (hi[i] - a + 4) & ~3, wsum[i], np);
 	}
 	if (threadIdx.x == 0) tlen[t] = (total + 3) / 4 * 4;   // lists start on 16-byte boundaries (bulk copies)
 }
@@ -1718,7 +1719,7 @@ __global__ void __launch_bounds__(RAYT_THREADS) k_tile_count(int ld, int H, int 
 // the tile's list (measurement indices in traced order) and its pixels'
 // 1-based positions in their part's stretch of it, padded with 0 to the warp's
 // word count
-__global__ void __launch_bounds__(RAYT_THREADS) k_tile_fill(int ld, int H, int ntx, int nrays,
+__global__ void __launch_bounds__(RAYT_THREADS) k_tile_fill(int ld, int H, int ntx, int nrays, int stride,
                                                             const int *__restrict__ cptr,
                                                             const int *__restrict__ cind,
                                                             const int *__restrict__ live_out,
@@ -1754,11 +1755,12 @@ __global__ void __launch_bounds__(RAYT_THREADS) k_tile_fill(int ld, int H, int n
 	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 	int k = p >= 0 ? cptr[p] : 0;
 	const int k1 = p >= 0 ? cptr[p + 1] : 0;
-	const int np = parts[t * TILE_PARTS].w;
+	parts += (long long)t * stride;
+	const int np = parts[0].w;
 	for (int i = 0; i < np; i++) {
-		const long long wl = ((long long)t * TILE_PARTS + i) * RAYT_WARPS + wid;
+		const long long wl = ((long long)t * stride + i) * RAYT_WARPS + wid;
 		const long long v0 = woff[wl];
-		const int nv = (int)((woff[wl + 1] - v0) >> 5), first = 1 - parts[t * TILE_PARTS + i].x;
+		const int nv = (int)((woff[wl + 1] - v0) >> 5), first = 1 - parts[i].x;
 		for (int v = 0; v < nv; v++, k += 8) {
 			int r[8];   // the word's eight loads first, then their positions
 #pragma unroll
@@ -1826,11 +1828,12 @@ static void upload_tiles(cudaStream_t s, std::vector<VTile> &vt, const std::vect
 }
 
 bool build_tiled_index(cudaStream_t s, int ld, int H, int nrays, const int *cptr, const int *cind,
-                       const int *live_out, OpDev &d, long long *bytes, std::vector<void *> &owned) {
+                       const int *live_out, OpDev &d, long long *bytes, long long *kept, std::vector<void *> &owned) {
 	if (nrays <= 0 || nrays > RAYT_MAX_RAYS) return false;
 	const int ntx = (ld + RAYT - 1) / RAYT, nty = (H + RAYT - 1) / RAYT, nt = ntx * nty;
-	const long long nw = (long long)nt * TILE_PARTS * RAYT_WARPS;
-	if (nt >= 1 << 24 || nw >= 1LL << 31) return false;
+	const bool cut = nt <= TILE_CUT;
+	const int stride = cut ? TILE_PARTS : 1;   // parts of a tile at most
+	const long long nw = (long long)nt * stride * RAYT_WARPS;
 	const int nwords = (nrays + 31) / 32;
 	const int smem = 2 * (int)sizeof(unsigned) * nwords;
 	// Each thread walks its own pixel's list of ray ids, so a warp touches 32
@@ -1848,19 +1851,19 @@ bool build_tiled_index(cudaStream_t s, int ld, int H, int nrays, const int *cptr
 	long long *tptr = (long long *)dev_alloc(sizeof(long long) * (nt + 1), s);
 	long long *wlen = (long long *)dev_alloc(sizeof(long long) * (nw + 1), s);
 	long long *woff = (long long *)dev_alloc(sizeof(long long) * (nw + 1), s);
-	int4 *parts = (int4 *)dev_alloc(sizeof(int4) * (size_t)nt * TILE_PARTS, s);
+	int4 *parts = (int4 *)dev_alloc(sizeof(int4) * (size_t)nt * stride, s);
 	unsigned char *perm = (unsigned char *)dev_alloc((size_t)nt * RAYT_THREADS, s);
 	// the tiles' ray bitmaps, kept from the count for the fill when they take
 	// at most 512 MB (else the fill builds them again)
 	const long long gbm_bytes = (long long)nt * nwords * (long long)sizeof(unsigned);
 	unsigned *gbm = gbm_bytes <= (512LL << 20) ? (unsigned *)dev_alloc((size_t)gbm_bytes, s) : nullptr;
-	k_tile_count<<<nt, RAYT_THREADS, smem, s>>>(ld, H, ntx, nrays, nt <= TILE_CUT ? TILE_PART : INT_MAX, cptr, cind, tlen, wlen,
+	k_tile_count<<<nt, RAYT_THREADS, smem, s>>>(ld, H, ntx, nrays, cut ? TILE_PART : INT_MAX, stride, cptr, cind, tlen, wlen,
 	                                            parts, perm, gbm);
 	TG_CUDA(cudaGetLastError());
 	scan_counts(s, tlen, tptr, nt);
 	scan_counts(s, wlen, woff, nw);
 	std::vector<long long> h_tptr(nt + 1);
-	std::vector<int4> h_parts((size_t)nt * TILE_PARTS);
+	std::vector<int4> h_parts((size_t)nt * stride);
 	long long words = 0;
 	TG_CUDA(cudaMemcpyAsync(h_tptr.data(), tptr, sizeof(long long) * (nt + 1), cudaMemcpyDeviceToHost, s));
 	TG_CUDA(cudaMemcpyAsync(h_parts.data(), parts, sizeof(int4) * h_parts.size(), cudaMemcpyDeviceToHost, s));
@@ -1874,12 +1877,12 @@ bool build_tiled_index(cudaStream_t s, int ld, int H, int nrays, const int *cptr
 			empty.push_back(t);
 			continue;
 		}
-		const int4 *q = &h_parts[(size_t)t * TILE_PARTS];
+		const int4 *q = &h_parts[(size_t)t * stride];
 		int live = 0, at = 0;
 		for (int i = 0; i < q[0].w; i++) live += q[i].y > 0;
 		for (int i = 0; i < q[0].w; i++)
 			if (q[i].y > 0) {
-				vt.push_back({t, at++, live, (int)(h_tptr[t] + q[i].x), q[i].y, q[i].z, (long long)t * TILE_PARTS + i});
+				vt.push_back({t, at++, live, (int)(h_tptr[t] + q[i].x), q[i].y, q[i].z, (long long)t * stride + i});
 				longest = std::max(longest, q[i].y);
 			}
 	}
@@ -1890,7 +1893,7 @@ bool build_tiled_index(cudaStream_t s, int ld, int H, int nrays, const int *cptr
 		uint4 *sidx = (uint4 *)dev_alloc(sizeof(uint4) * (size_t)std::max(words, 1LL), s);
 		int *woff32 = (int *)dev_alloc(sizeof(int) * (nw + 1), s);
 		owned.push_back(tmeas); owned.push_back(sidx); owned.push_back(woff32); owned.push_back(perm);
-		k_tile_fill<<<nt, RAYT_THREADS, smem, s>>>(ld, H, ntx, nrays, cptr, cind, live_out, tptr, woff, parts, perm, tmeas,
+		k_tile_fill<<<nt, RAYT_THREADS, smem, s>>>(ld, H, ntx, nrays, stride, cptr, cind, live_out, tptr, woff, parts, perm, tmeas,
 		                                           sidx, gbm);
 		TG_CUDA(cudaGetLastError());
 		k_to_int<<<(unsigned)((nw + 1 + 255) / 256), 256, 0, s>>>(woff, woff32, nw + 1);
@@ -1898,6 +1901,7 @@ bool build_tiled_index(cudaStream_t s, int ld, int H, int nrays, const int *cptr
 		*bytes = (long long)sizeof(uint4) * words + (long long)sizeof(int) * (h_tptr[nt] + (long long)vt.size() * RAYT_WARPS) +
 		         (long long)nt * RAYT_THREADS;
 		upload_tiles(s, vt, empty, nt, d, owned, bytes);
+		*kept = *bytes + (long long)sizeof(int) * (nw + 1 - (long long)vt.size() * RAYT_WARPS);   // offsets of parts that are not there
 		d.ntx = ntx;
 		d.nty = nty;
 		d.tmeas = tmeas; d.woff = woff32; d.sidx = sidx; d.tperm = perm;
@@ -2142,7 +2146,7 @@ bool build_brick_words(cudaStream_t s, int rvx, int rvy, int rvz, const int *cpt
 
 #else   // FP64 build: the ray adjoints are the pixel-major gathers
 bool build_tiled_index(cudaStream_t, int, int, int, const int *, const int *, const int *, OpDev &, long long *,
-                       std::vector<void *> &) {
+                       long long *, std::vector<void *> &) {
 	return false;
 }
 int tiled_smem_bytes(int) { return 0; }

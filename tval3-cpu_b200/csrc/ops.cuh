@@ -96,11 +96,12 @@ constexpr int ATOMIC_ZERO_TILE = 1024;
 // the tiled 2D ray adjoint's index (OpDev::tiled) for an ld x H image, from
 // the pixel-major lists of traced-ray ids (cptr, cind; sorted by ray) and the
 // measurement index of every traced ray.  Fills d's tiled fields, allocates
-// the index (recorded in `owned`, its size stored in *bytes) and returns true;
-// returns false, allocating nothing, when there are more than RAYT_MAX_RAYS
-// traced rays or a tile list would exceed RAYT_MAX_LIST.
+// the index (recorded in `owned`; *bytes: what an adjoint reads of it, *kept: its
+// size) and returns true; returns false, allocating nothing, when there are more
+// than RAYT_MAX_RAYS traced rays or the list of a tile, or of a part of one,
+// would exceed RAYT_MAX_LIST.
 bool build_tiled_index(cudaStream_t s, int ld, int H, int nrays, const int *cptr, const int *cind,
-                       const int *live_out, OpDev &d, long long *bytes, std::vector<void *> &owned);
+                       const int *live_out, OpDev &d, long long *bytes, long long *kept, std::vector<void *> &owned);
 int tiled_smem_bytes(int tmax);
 
 // The same tiled adjoint for 3D rays, over bricks of BRICK_X x BRICK_Y x

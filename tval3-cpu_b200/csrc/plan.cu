@@ -417,9 +417,9 @@ void prepare_op(cudaStream_t s, const tval3g_problem &p, int flags, OpStore &st,
 		if (!is3 && n % p.ld == 0 && d.nrays > 0 && d.nrays <= RAYT_MAX_RAYS && tile_ok) {
 			// tiled adjoint (cind still holds traced-ray ids)
 			const int *lo = dout;
-			long long ib = 0;
-			if (build_tiled_index(s, (int)p.ld, (int)(n / p.ld), d.nrays, cptr, cind, lo, d, &ib, st.owned)) {
-				st.bytes += ib;
+			long long ib = 0, kept = 0;
+			if (build_tiled_index(s, (int)p.ld, (int)(n / p.ld), d.nrays, cptr, cind, lo, d, &ib, &kept, st.owned)) {
+				st.bytes += kept;
 				st.adj_index_bytes = ib;
 				if (const char *e = std::getenv("TVAL3G_TEST_FIRST_WAIT_POLLS"))   // failure-path test hook
 					d.first_wait_polls = 1u + (unsigned)std::strtoul(e, nullptr, 10);
