@@ -469,7 +469,7 @@ private:
 	size_t arena_off_ = 0;
 	void layout();
 	double *da(long long count);
-	ChunkState state_alloc();
+	ChunkState state_alloc(bool own_r = true);   // false: r goes to rb_, which a forward does not use
 	void release();
 	Rows rows(bool trans, const double *x) const;
 	int row_blocks(bool trans) const;
@@ -487,6 +487,7 @@ void Unrolled::layout() {
 	nbp_ = (int)std::min<long long>(EW_BLOCKS, (n_ * W_ + EW_THREADS - 1) / EW_THREADS);
 	ch_.clear();
 	seg_.clear();
+	rb_ = da(m_ * W_);
 	const int nck = (K_ - 1) / C_ + 1;   // segments: states 0, C, 2 C, ... below K start one
 	for (int f = 0; f < count_; f += W_) {
 		Chunk c;
@@ -496,14 +497,16 @@ void Unrolled::layout() {
 		c.steps = da((long long)K_ * W_);
 		c.outer = reinterpret_cast<int *>(da((long long)K_ * W_));
 		for (int k = 0; k < nck; k++) {
-			c.ck.push_back(state_alloc());
+			// r is read of iteration 0's state alone: the later ones, which end a
+			// segment too, are recomputed as its last state
+			c.ck.push_back(state_alloc(k == 0));
 			c.ckd.push_back(da(n_ * W_));
 		}
 		ch_.push_back(c);
 	}
 	for (int j = 0; j < std::max(2, std::min(C_, K_)); j++) seg_.push_back(state_alloc());
 	for (double **v : {&dbuf_[0], &dbuf_[1], &t_, &ub_, &sbx_, &sby_, &dd_, &vbx_, &vby_}) *v = da(n_ * W_);
-	for (double **v : {&q_meas_, &dlb_, &bsb_, &rb_}) *v = da(m_ * W_);
+	for (double **v : {&q_meas_, &dlb_, &bsb_}) *v = da(m_ * W_);
 	pp_ = da((long long)(K_ + 1) * nbp_ * NPIX);
 	pm_ = da((long long)(K_ + 1) * nbm_ * NMEAS);
 	sums_ = da((long long)(K_ + 1) * (NPIX + NMEAS));
@@ -636,13 +639,13 @@ void Unrolled::release() {
 
 #define EW(kern, grid, ...) launch_pdl(kern, dim3(grid), dim3(EW_THREADS), 0, s, __VA_ARGS__)
 
-ChunkState Unrolled::state_alloc() {
+ChunkState Unrolled::state_alloc(bool own_r) {
 	ChunkState t;
 	t.U = da(n_ * W_);
 	t.sx = da(n_ * W_);
 	t.sy = da(n_ * W_);
 	t.dl = da(m_ * W_);
-	t.r = da(m_ * W_);
+	t.r = own_r ? da(m_ * W_) : rb_;
 	return t;
 }
 
