@@ -207,6 +207,11 @@ int tval3g_plan_stats(const tval3g_plan *plan, long long *kernel_launches, long 
  * plan's state (the next solve starts afresh).  No counterpart in the
  * reference. */
 int tval3g_plan_time_stencils(tval3g_plan *plan, int reps, double *ms);
+/* The same for the one kernel in which an iteration on real data takes the
+ * gradient epilogue and the shrinkage together: *ms; 0 for plans that launch
+ * them one after the other (complex data; image vectors above 32 GB), as every
+ * plan does at its start and after a line search. */
+int tval3g_plan_time_step(tval3g_plan *plan, int reps, double *ms);
 /* Time-to-solution mode: with target > 0, every instance solved with a Ut
  * also stops after the first inner iteration at which
  * ||U/scl - Ut|| <= target * ||Ut|| (checked on the device each iteration);

@@ -81,3 +81,21 @@ def test_plan_above_32_gb(tv, torch_cuda):
     del Ul, part
     torch.cuda.empty_cache()
     capi.trim_memory()
+
+
+def test_time_step(torch_cuda):
+    """The iteration's one kernel is timed where the plan runs it, and 0 elsewhere; the next solve starts afresh."""
+    torch = torch_cuda
+    m, n, rowptr, colind, val, A, b = problem((23, 31), 1)
+    opts = W.options(2.0 ** 6, 2.0 ** 4, 1e-9, 4)
+    spec = capi.csr_problem((23, 31), m, n, rowptr, colind, val)
+    plan = capi.Plan([spec], [opts])
+    db, u1, u2 = [torch.tensor(b, device="cuda")], [torch.empty(n, device="cuda")], [torch.empty(n, device="cuda")]
+    plan.solve(db, u1)
+    assert plan.time_step(5) > 0
+    plan.solve(db, u2)
+    assert torch.equal(u1[0], u2[0])
+    plan.close()
+    cplx = capi.Plan([capi.csr_problem((23, 31), m, n, rowptr, colind, val.astype(np.complex64))], [opts])
+    assert cplx.time_step(5) == 0
+    cplx.close()

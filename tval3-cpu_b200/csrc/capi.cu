@@ -198,7 +198,15 @@ int tval3g_plan_stats(const tval3g_plan *plan, long long *kernel_launches, long 
 int tval3g_plan_time_stencils(tval3g_plan *plan, int reps, double *ms) {
 	CAPI_BEGIN
 	TG_ARG(plan && plan->p && ms && reps >= 1, "Argument error: NULL plan or output, or reps < 1");
-	plan->p->time_stencils(reps, ms);
+	plan->p->time_stencils(reps, ms, false);
+	CAPI_END
+}
+
+int tval3g_plan_time_step(tval3g_plan *plan, int reps, double *ms) {
+	CAPI_BEGIN
+	TG_ARG(plan && plan->p && ms && reps >= 1, "Argument error: NULL argument or reps < 1");
+	*ms = 0;
+	if (plan->p->fused_step()) plan->p->time_stencils(reps, ms, true);
 	CAPI_END
 }
 

@@ -860,7 +860,7 @@ Plan::Plan(int count, const tval3g_problem *probs, const tval3g_options *opts, i
 
 Plan::~Plan() { release(); }
 
-void Plan::time_stencils(int reps, double ms[3]) {
+void Plan::time_stencils(int reps, double *ms, bool step) {
 	cur_ = stream_;
 	const bool gm = graph_mode_;
 	graph_mode_ = false;   // es() is the launch stream
@@ -868,9 +868,10 @@ void Plan::time_stencils(int reps, double ms[3]) {
 	try {
 		TG_CUDA(cudaEventCreate(&e0));
 		TG_CUDA(cudaEventCreate(&e1));
-		for (int k = 0; k < 3; k++) {
+		for (int k = 0; k < (step ? 1 : 3); k++) {
 			auto launch = [&] {
-				if (k == 0) launch_getg(stream_, kargs(MAP_NM, P_ALL, ST_DESCEND));
+				if (step) launch_getg_shrink(stream_, kargs(MAP_NM, P_ALL, ST_DESCEND));
+				else if (k == 0) launch_getg(stream_, kargs(MAP_NM, P_ALL, ST_DESCEND));
 				else if (k == 1) launch_descend(stream_, kargs(MAP_NM, P_ALL, ST_DESCEND));
 				else launch_shrink_grad(stream_, kargs(MAP_N, P_ALL, ST_LOOP));
 			};

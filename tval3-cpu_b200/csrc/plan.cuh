@@ -69,7 +69,8 @@ public:
 	// mean device time (ms) of one launch of k_getg (descent stage), k_descend
 	// (descent stage) and k_shrink_grad over every instance, each launched reps
 	// times back to back after the last solve (whose state they overwrite)
-	void time_stencils(int reps, double ms[3]);
+	bool fused_step() const { return fused_step_; }
+	void time_stencils(int reps, double *ms, bool step);   // three kernels, or (step) k_getg_shrink alone
 
 private:
 	struct Frame {

@@ -87,6 +87,7 @@ def lib():
         L.tval3g_plan_trace.argtypes = [vp, i, C.POINTER(C.c_double), i, C.POINTER(i)]
         L.tval3g_plan_set_target.argtypes = [vp, d]
         L.tval3g_plan_time_stencils.argtypes = [vp, i, C.POINTER(d)]
+        L.tval3g_plan_time_step.argtypes = [vp, i, C.POINTER(d)]
         L.tval3g_plan_destroy.argtypes = [vp]
         L.tval3g_trim_memory.argtypes = [ll]
         L.tval3g_tune_stats.argtypes = [C.POINTER(ll), C.POINTER(ll)]
@@ -148,7 +149,7 @@ def tune_stats():
 EXPORTS = ("tval3g_last_error", "tval3g_version", "tval3g_solve", "tval3g_solve_f64", "tval3g_solve_batch",
            "tval3g_plan_create",
            "tval3g_plan_solve", "tval3g_plan_stats", "tval3g_plan_trace", "tval3g_plan_set_target",
-           "tval3g_plan_time_stencils",
+           "tval3g_plan_time_stencils", "tval3g_plan_time_step",
            "tval3g_plan_destroy", "tval3g_trim_memory", "tval3g_tune_stats", "tval3g_op_launch_shape",
            "tval3g_op_create", "tval3g_op_shape",
            "tval3g_op_apply", "tval3g_op_apply_n", "tval3g_op_ray_csr", "tval3g_op_adjoint_index_bytes",
@@ -359,6 +360,14 @@ class Plan:
         ms = (C.c_double * 3)()
         _check(lib().tval3g_plan_time_stencils(self.h, int(reps), ms))
         return {"getg": ms[0], "descend": ms[1], "shrink_grad": ms[2]}
+
+    def time_step(self, reps=20):
+        """Mean ms per launch of the one kernel for the gradient epilogue and
+        the shrinkage, as iterations on real data run them; 0.0 where they are
+        two launches.  As time_stencils otherwise."""
+        ms = C.c_double()
+        _check(lib().tval3g_plan_time_step(self.h, int(reps), C.byref(ms)))
+        return ms.value
 
     def stats(self):
         a, b = C.c_longlong(), C.c_longlong()
