@@ -1369,14 +1369,16 @@ constexpr int RAYT_LIST_CHUNK = 8192;                    // list entries per bul
 // 18.1 25.7 19.8; 8192: 13.5 15.1 19.7 16.8; 6144: 11.3 14.1 17.5 15.9; 4096:
 // 10.6 17.1 18.8 16.4.  Of (256, 512), 256 tiles: whole 26.0, 8192 rays 25.6
 // with the index in L2 but 5 % slower with it from HBM.
+// (The image's tiles count, not the launch's: parts add in another order, and an
+// instance gives the same bits alone and in a batch.)
 constexpr int TILE_PART = 6144, TILE_CUT = 148;
 static_assert(TILE_CUT < 1 << 24, "tile numbers beside part numbers (OpDev::vtile)");
 constexpr int TILE_PARTS = 16;                           // parts per tile at most
 constexpr int RAYT_ZERO_TILES = 16;                      // tiles without rays zeroed per block
 
-// barrier, second-half sums, then the tile's measurements: slot 0 (the zero
-// pad entries read) sits 12 bytes past a 16-byte boundary so that slots 1..
-// are aligned for the bulk copy of the list
+// the list's barrier and the pixel-warps' word offsets, the runs' sums, then the
+// list's measurements: slot 0 (the zero that pad entries read) sits 12 bytes past
+// a 16-byte boundary so that slots 1.. are aligned for the bulk copy of the list
 int tiled_smem_bytes(int tmax) {
 	return RAYT_BAR_BYTES + RAYT_SACC_BYTES + 12 + (int)sizeof(float) * (tmax + 1);
 }
@@ -1394,6 +1396,22 @@ __device__ __forceinline__ uint4 ld_word(const uint4 *p) {
 __device__ __forceinline__ float word_sum(const float *yt, uint4 q) {
 	return ((yt[q.x & 0xffff] + yt[q.x >> 16]) + (yt[q.y & 0xffff] + yt[q.y >> 16])) +
 	       ((yt[q.z & 0xffff] + yt[q.z >> 16]) + (yt[q.w & 0xffff] + yt[q.w >> 16]));
+}
+
+// g at pixel px (0 .. RAYT^2 - 1, row-major in the tile) of tile (brick) t
+__device__ __forceinline__ void tiled_store(const Inst &I, const OpDev &op, VecSel ys, int t, int px, float v) {
+	if (op.tile3) {   // brick of BRICK_X x BRICK_Y x BRICK_Z voxels
+		const int bxy = op.ntx * op.nty;
+		const int x = (t % op.ntx) * BRICK_X + px % BRICK_X;
+		const int y = ((t % bxy) / op.ntx) * BRICK_Y + (px / BRICK_X) % BRICK_Y;
+		const int z = (t / bxy) * BRICK_Z + px / (BRICK_X * BRICK_Y);
+		// (the last layer of bricks may reach beyond the image's end, where the volume is smaller than the image)
+		const long long p = x + (long long)y * op.rvx + (long long)z * op.rvx * op.rvy;
+		if (x < op.rvx && y < op.rvy && p < I.n) vselw(I, ys)[p] = v;
+		return;
+	}
+	const int x = (t % op.ntx) * RAYT + (px % RAYT), row = (t / op.ntx) * RAYT + (px / RAYT);
+	if (x < op.rvx && row < op.tH) vselw(I, ys)[x + row * op.rvx] = v;
 }
 
 // g[p] = scale * sum over the rays through p of y[ray] (the transposed
@@ -1417,22 +1435,6 @@ __device__ __forceinline__ float word_sum(const float *yt, uint4 q) {
 // equal runs.  256^2 ring: 32.4 -> 25.8 us (225 blocks on 148 SMs).
 // Lists in the forward's sorted ray order (y permuted first) took 174 us there
 // but 16.0 against 13.0 us at 64^3 and 44.5 against 42.3 at 100^3: not kept.
-// g at pixel px (0 .. RAYT^2 - 1, row-major in the tile) of tile (brick) t
-__device__ __forceinline__ void tiled_store(const Inst &I, const OpDev &op, VecSel ys, int t, int px, float v) {
-	if (op.tile3) {   // brick of BRICK_X x BRICK_Y x BRICK_Z voxels
-		const int bxy = op.ntx * op.nty;
-		const int x = (t % op.ntx) * BRICK_X + px % BRICK_X;
-		const int y = ((t % bxy) / op.ntx) * BRICK_Y + (px / BRICK_X) % BRICK_Y;
-		const int z = (t / bxy) * BRICK_Z + px / (BRICK_X * BRICK_Y);
-		// (the last layer of bricks may reach beyond the image's end, where the volume is smaller than the image)
-		const long long p = x + (long long)y * op.rvx + (long long)z * op.rvx * op.rvy;
-		if (x < op.rvx && y < op.rvy && p < I.n) vselw(I, ys)[p] = v;
-		return;
-	}
-	const int x = (t % op.ntx) * RAYT + (px % RAYT), row = (t / op.ntx) * RAYT + (px / RAYT);
-	if (x < op.rvx && row < op.tH) vselw(I, ys)[x + row * op.rvx] = v;
-}
-
 __global__ void __launch_bounds__(RAYT_ADJ_THREADS, 2) k_ray_adj_tiled(const Inst *tab, TileMap map, int pred,
                                                                        VecSel xs, VecSel ys, int *err,
                                                                        unsigned long long *launches) {
@@ -2395,9 +2397,9 @@ __global__ void k_entry_rows(long long rows, const int *rptr, int *row_of) {
 	for (int k = rptr[row] + lane; k < rptr[row + 1]; k += 32) row_of[k] = (int)row;
 }
 
-// digit counts of one tile of entries: hist[digit * tiles + tile]
-// digit counts of one tile: one add for a warp whose entries share their digit
-// (as those of a ray along y, low digit, or x, high digit, do), else one each;
+// digit counts of one tile of entries, hist[digit * tiles + tile]: one add for a
+// warp whose entries share their digit (as those of a ray along y, low digit, or
+// x, high digit, do), else one each;
 // 27M entries of the 256^2 ring's 130816 rays: 57 -> 36 us.  (The warp's groups
 // of equal digits by eight ballots: 106; by match.any: 145.)
 __global__ void __launch_bounds__(RADIX_T) k_radix_hist(const int *__restrict__ key, long long nnz, int shift,

@@ -77,8 +77,9 @@ struct OpBatch {
 	// its mean line length (4, 8, 16 or 32 lanes per line: class 0..3), so its
 	// summation order does not depend on the other instances of a batch.
 	TileMap csr_fwd[4], csc_adj[4], ray_adj[4];
-	// rays: on-the-fly Bresenham, 4, 8 or 16 lanes per ray (class 0..2;
-	// RAY_SUBW = 8 unless the autotuner chose otherwise), 2D and 3D
+	// rays: on-the-fly Bresenham, 4, 8 or 16 lanes per ray or one thread (classes
+	// 0..3, RAY_LANES; one thread or RAY_SUBW = 8 lanes by the launch's rays unless
+	// the autotuner chose otherwise), 2D and 3D
 	TileMap ray2_fwd[4], ray3_fwd[4];
 	// 32x32 tiles of the image (of the slices of the volume), for ray operators with xT
 	TileMap ray2_transpose, ray3_transpose;
