@@ -1143,9 +1143,9 @@ __global__ void __launch_bounds__(256) k_ray_fwd(const Inst *tab, TileMap map, i
 // sums in FP64 per class, the classes in the shuffle tree's order.
 // Bound: 2D by issue (7 warp instructions per hit and lane, 18 before) at 28
 // resident warps per SM - 256^2 ring, 2.72e7 hits, with the transpose: 26.0 ->
-// 15.8 us; 3D by L2 (a warp's hits spread over about 12 sectors, read once) -
-// 128^3 hemisphere, 1.29e8 hits, with the transpose: 295 -> 147 us, L2 at 70 %
-// of its throughput.
+// 15.8 us; 3D by L1's rate of lines and the latency of its L2 hits (a warp's hits
+// spread over about 12 sectors, read once; L1 77 % busy, L2 71, issue 45) -
+// 128^3 hemisphere, 1.29e8 hits, with the transpose: 295 -> 147 us.
 template <bool D3>
 __global__ void __launch_bounds__(RAY1_BLOCK) k_ray_fwd_thread(const Inst *tab, TileMap map, int pred, VecSel xs,
                                                                VecSel ys, unsigned long long *launches) {
