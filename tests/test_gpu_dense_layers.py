@@ -41,6 +41,23 @@ def test_layers_equal_one_right_hand_side(m, h, w, layers, torch_cuda):
     many.close()
 
 
+@pytest.mark.parametrize("m,h,w", [(20000, 16, 32), (20001, 16, 32), (90000, 4, 4), (30000, 63, 65), (30000, 64, 64)])
+def test_normal_product_of_many_short_rows(m, h, w, torch_cuda):
+    """Both sides of the line from which it is two products (rows of fewer than 4096 columns)."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(m)
+    A = torch.randn((m, h * w), generator=g, device="cuda") / 64
+    x = torch.randn(h * w, generator=g, device="cuda")
+    op = capi.Operator(capi.dense_problem((h, w), A, device_ptr=A.data_ptr()), device_inputs=True)
+    y = op.apply(x, torch.full((h * w,), 7.0, device="cuda"), trans=2)
+    A64, B64 = A.double(), A.double().abs()
+    want = A64.T @ (A64 @ x.double())
+    # A x rounded (by rows: eight products in FP32 first), float partials of row chunks, one rounding
+    assert bool(((y.double() - want).abs() <= 16 * 2.0 ** -24 * (B64.T @ (B64 @ x.double().abs()))).all())
+    assert float((y.double() - want).norm() / want.norm()) < 3e-7
+    op.close()
+
+
 def test_matrix_not_16_byte_aligned(torch_cuda):
     torch = torch_cuda
     g = torch.Generator(device="cuda").manual_seed(3)

@@ -38,8 +38,8 @@ TG_BEGIN
 // aligned, has x converted once per block, chunk by chunk into shared memory.
 // The segments of 32 elements (float4s) that a row is read in go to CLASSES
 // classes in turn - four, fewer for long rows; lane l adds the l-th products of
-// a class in order, the lanes are added by halves, then the classes: the same
-// bits in a launch of few rows and of many.
+// a class in order, then its classes' sums, then the lanes are added by halves:
+// the same bits in a launch of few rows and of many.
 // Bound: the float-to-double conversions (two a product; with x in shared memory
 // one), A from memory where it is larger than L2; for few rows the loads in
 // flight.  Measured, us (one warp a row in one class, straight from memory -> this):
@@ -169,53 +169,40 @@ template <int WPR, int CLASSES>
 struct DenseRow {
 	static constexpr int NC = CLASSES / WPR;   // classes of a warp: sub, sub + WPR, ...
 	int n, sub;   // this warp: part sub of the row
-	unsigned row, layer;
-	const real *a, *x;   // (rows beyond the last: the last again, not stored)
+	int out;             // its element of y; -1: beyond the last row (which is read again, not stored)
+	const real *a, *x;
 	double acc[NC] = {};
 	__device__ __forceinline__ DenseRow(const Inst &I, const VecSel &xs, int local) {
 		constexpr unsigned ROWS = WARPS / WPR;
 		const unsigned m = (unsigned)I.op.m, rt = (m + ROWS - 1) / ROWS, warp = threadIdx.x >> 5;
 		n = (int)I.op.n;
 		sub = (int)(warp % WPR);
-		layer = (unsigned)local / rt;
-		row = ((unsigned)local - layer * rt) * ROWS + warp / WPR;
+		const unsigned layer = (unsigned)local / rt, row = ((unsigned)local - layer * rt) * ROWS + warp / WPR;
+		out = row < m ? (int)(layer * m + row) : -1;
 		a = I.op.A + (long long)min(row, m - 1) * n;
 		x = vsel(I, xs) + (long long)layer * n;
 	}
-	// y = the classes' sums over the lanes, added in order.  Class k's ends in
-	// lane k 32 / NC: at each level a lane gives away half of the classes that it
-	// still has (as warp_sums does).
+	// y = the lanes' sums of the classes, in order, then the lanes by halves; the
+	// warps of a row meet in shared memory before that
 	__device__ __forceinline__ void store(const Inst &I, const VecSel &ys) {
 		const int lane = threadIdx.x & 31;
-#pragma unroll
-		for (int h = NC / 2, o = 16; h > 0; h >>= 1, o >>= 1) {
-			const bool up = lane & o;
-#pragma unroll
-			for (int k = 0; k < h; k++) {
-				const double give = up ? acc[k] : acc[k + h], keep = up ? acc[k + h] : acc[k];
-				acc[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-			}
-		}
-		double s = acc[0];
-#pragma unroll
-		for (int o = 16 / NC; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-		double t = 0.0;
+		double t = acc[0];
 		if (WPR == 1) {
-			t = s;
 #pragma unroll
-			for (int k = 1; k < CLASSES; k++) t += __shfl_sync(0xffffffffu, s, k * (32 / NC));
+			for (int k = 1; k < CLASSES; k++) t += acc[k < NC ? k : 0];
 		} else {
-			__shared__ double ws[WARPS / WPR][CLASSES];
-			double *w = ws[(threadIdx.x >> 5) / WPR];
-			if (lane % (32 / NC) == 0) w[lane / (32 / NC) * WPR + sub] = s;
-			__syncthreads();
-			if (sub == 0 && lane == 0) {
-				t = w[0];
+			__shared__ double ws[WARPS / WPR][CLASSES][32];
+			double(*w)[32] = ws[(threadIdx.x >> 5) / WPR];
 #pragma unroll
-				for (int k = 1; k < CLASSES; k++) t += w[k];
-			}
+			for (int k = 0; k < NC; k++) w[k * WPR + sub][lane] = acc[k];
+			__syncthreads();
+			if (sub) return;
+			t = w[0][lane];
+#pragma unroll
+			for (int k = 1; k < CLASSES; k++) t += w[k][lane];
 		}
-		if (sub == 0 && lane == 0 && row < I.op.m) vselw(I, ys)[layer * I.op.m + row] = (real)t;
+		t = warp_sum(t);
+		if (lane == 0 && out >= 0) vselw(I, ys)[out] = (real)t;
 	}
 };
 

@@ -26,6 +26,12 @@ inline DenseForm dense_form(long long rows, long long n, bool vec) {
 	if (few) return DENSE_FOUR;
 	return !vec && n >= DENSE_CHUNK && !FP64_BUILD ? DENSE_SHORT : DENSE_ONE;
 }
+// matrices whose normal product is the two gemv products: many short rows, where
+// the one-pass forms are a chain of barriers per row (by rows / by bands / two
+// products, us: 100000 x 256 549, 512, 100; 40000 x 1024 225, 222, 77; 70000 x
+// 2000 392, 378, 228; below, by rows gains or the latencies are alike: 300 x 1024
+// 8.2, 20.8, 13)
+inline bool dense_tall(long long m, long long n) { return m > 20000 && n < 4096; }
 inline int dense_form_rows(DenseForm f) { return f == DENSE_FOUR ? 2 : f == DENSE_LONG_TWO ? 4 : 8; }   // per block
 
 // lanes per ray of the on-the-fly forward projectors where there are few rays

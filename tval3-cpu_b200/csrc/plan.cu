@@ -507,7 +507,7 @@ static long long build_op_maps(std::vector<Inst> &inst, const std::vector<OpStor
 	for (int i = 0; i < cnt; i++) {
 		OpDev &d = inst[i].op;
 		d.fused_rpc = 0;
-		if (d.kind != TVAL3G_OP_DENSE || d.mrhs || d.layers != 1) continue;
+		if (d.kind != TVAL3G_OP_DENSE || d.mrhs || d.layers != 1 || dense_tall(d.m, d.n)) continue;
 		if (fused_by_rows(d.m, d.n, d.A)) {
 			d.fused_rpc = 1;   // (marks it as fused)
 			ob.fused.push_back({i, 0, 0, d.n, fused_rows_grid(d.n)});
