@@ -237,8 +237,8 @@ int tval3g_tune_stats(long long *measured, long long *cached);
 /* Operators alone.  tval3g_op_apply: y = A x (trans = 0), y = A^T x
  * (trans = 1) or the normal product y = A^T (A x) of the solve's get_g_mult
  * (trans = 2; a one-layer dense operator - unless of very many short rows -
- * reads A once, as the reference's
- * cache-blocked dense path, 2d/tval3_cpu_2d.cpp:361-394) with DEVICE x, y
+ * reads A once, as the reference's cache-blocked dense path,
+ * 2d/tval3_cpu_2d.cpp:361-394) with DEVICE x, y
  * (lengths rows/cols as reported; both cols for trans = 2).  An operator keeps
  * scratch for its products (partial sums, transposed images): products of one
  * operator must not overlap on the device.  Enqueue them on one stream, or

@@ -27,9 +27,11 @@ inline DenseForm dense_form(long long rows, long long n, bool vec) {
 	return !vec && n >= DENSE_CHUNK && !FP64_BUILD ? DENSE_SHORT : DENSE_ONE;
 }
 // matrices whose normal product is the two gemv products: many short rows, where
-// the one-pass forms are a chain of barriers per row (by rows / by bands / two
-// products, us: 100000 x 256 549, 512, 100; 40000 x 1024 225, 222, 77; 70000 x
-// 2000 392, 378, 228; below, by rows gains or the latencies are alike: 300 x 1024
+// the one-pass forms are a chain of barriers per row.  The line lies where the
+// form by rows falls behind the one by bands (by rows / by bands / two products,
+// us: 100000 x 256 549, 512, 100; 40000 x 1024 225, 222, 70; 30000 x 512 169, 165,
+// 36); between it and some 3000 rows two products would win too (20000 x 512 115,
+// 116, 28; 5000 x 1024 33, 46, 21), below and for wider rows they lose (300 x 1024
 // 8.2, 20.8, 13)
 inline bool dense_tall(long long m, long long n) { return m > 20000 && n < 4096; }
 inline int dense_form_rows(DenseForm f) { return f == DENSE_FOUR ? 2 : f == DENSE_LONG_TWO ? 4 : 8; }   // per block
