@@ -907,16 +907,33 @@ int fused_rows_per_cta(long long, long long, int, const real *, int *) { return 
 bool fused_by_rows(long long, long long, const real *) { return false; }
 int fused_rows_grid(long long) { return 1; }
 #endif
+// Kernels that read the instance and its index, which no kernel of a chain
+// writes, before they wait for the previous kernel (the caller's own arrays only
+// after it: the previous kernel may be the caller's)
+#define RAY_PROLOGUE()                                                                \
+	pdl_launch_next();                                                                \
+	if (launches && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(launches, 1ull);   \
+	const int2 tl_ = map.tiles[blockIdx.x];                                           \
+	const Inst &I = tab[tl_.x];                                                       \
+	const OpDev &op = I.op;
+#define RAY_WAIT()                                                                    \
+	pdl_wait_prev();                                                                  \
+	if (!pred_ok(*I.ctrl, pred)) return;
+
 // ---------------------------------------------------------------------------
 // compressed gather: y[line] = w * sum_k val[k] * x[ind[k]] over a line's range
 //   kind 0: CSR rows (forward), kind 1: CSC columns (adjoint of CSR),
 //   kind 2: ray adjoint (implicit weight = scale, ind = measurement index)
+// Small operators are bound by the chain of loads from the instance to the first
+// entry, so what no kernel writes of it is read before the wait (us a product,
+// before: sparse 97x97 adjoint 6.8 -> 5.5, forward 6.1 -> 5.4, 40x40 4.5 -> 3.5, 160x160
+// 13.6 -> 12.5); large ones by the L2's sectors (hemisphere of 32^3 voxels and
+// 1.6M rays 80 -> 77.4).
 // ---------------------------------------------------------------------------
 template <int W>
 __global__ void __launch_bounds__(256) k_gather(const Inst *tab, TileMap map, int pred, int kind, VecSel xs,
                                                 VecSel ys, unsigned long long *launches) {
-	OPROLOGUE();
-	const OpDev &op = I.op;
+	RAY_PROLOGUE();
 	const int *ptr, *ind;
 	const real *val;
 	long long lines, xlen, ylen;
@@ -924,16 +941,25 @@ __global__ void __launch_bounds__(256) k_gather(const Inst *tab, TileMap map, in
 	else if (kind == 1) { ptr = op.cptr; ind = op.cind; val = op.cval; lines = op.n; xlen = op.m; ylen = op.n; }
 	else { ptr = op.cptr; ind = op.cind; val = nullptr; lines = I.n; xlen = 0; ylen = 0; }
 	constexpr int LPB = 256 / W;   // lines per block
-	const long long lt = (lines + LPB - 1) / LPB;
-	const long long layer = local / lt;
-	const long long line = (local - layer * lt) * LPB + threadIdx.x / W;
+	const unsigned local = (unsigned)tl_.y, lt = (unsigned)((lines + LPB - 1) / LPB), layer = local / lt;
+	const long long line = (long long)(local - layer * lt) * LPB + threadIdx.x / W;
 	const int gl = threadIdx.x % W;
+	// the line's range before the wait, unless the CSR may be the caller's
+	int k0 = 0, k1 = 0;
+	auto range = [&]() {
+		if (line < lines) {
+			k0 = ptr[line];
+			k1 = ptr[line + 1];
+		}
+	};
+	if (kind) range();
+	RAY_WAIT();
+	if (!kind) range();
 	const real *x = vsel(I, xs) + layer * xlen;
 	double acc = 0.0;   // FP64 accumulation of FP32 products
 	if (line < lines) {
 		// four of the lane's entries per step: their indices, then the four
 		// gathers, in flight together; summed in the lane's entry order
-		const int k0 = ptr[line], k1 = ptr[line + 1];
 		int k = k0 + gl;
 		if (val) {
 			for (; k + 3 * W < k1; k += 4 * W) {
@@ -1014,18 +1040,6 @@ struct MinorStep {
 		if (r >= twoM) { r -= twoM; q++; }
 	}
 };
-
-// The forward projections unpack their rays and set up the stepping before
-// they wait for the previous kernel: none of it depends on one.
-#define RAY_PROLOGUE()                                                                \
-	pdl_launch_next();                                                                \
-	if (launches && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(launches, 1ull);   \
-	const int2 tl_ = map.tiles[blockIdx.x];                                           \
-	const Inst &I = tab[tl_.x];                                                       \
-	const OpDev &op = I.op;
-#define RAY_WAIT()                                                                    \
-	pdl_wait_prev();                                                                  \
-	if (!pred_ok(*I.ctrl, pred)) return;
 
 // Forward projection, SUBW lanes per ray.  Lane l takes the hits j = l,
 // l + SUBW, ...; the linear index advances by SUBW driving steps plus, per
