@@ -1,6 +1,7 @@
 // Measurement operators of the TVAL3 solve (modk/tval3-cpu 2d/mat_mult.h,
 // 3d/mat_mult.h), batched over the instances of a plan.
 #pragma once
+#include <algorithm>
 #include <vector>
 #include <memory>
 #include <utility>
@@ -37,7 +38,7 @@ inline bool dense_tall(long long m, long long n) { return m > 20000 && n < 4096;
 inline int dense_form_rows(DenseForm f) { return f == DENSE_FOUR ? 2 : f == DENSE_LONG_TWO ? 4 : 8; }   // per block
 
 // lanes per ray of the on-the-fly forward projectors where there are few rays
-// (below RAY1_MIN_RAYS): a warp traces 32 / RAY_SUBW rays at once, which spreads
+// (below RAY1_MIN_RAYS, ray1_min_rays_3d): a warp traces 32 / RAY_SUBW rays at once, which spreads
 // the per-ray set-up (unpacking, the closed-form start of every lane, the final
 // shuffle sum) over several rays; 2D rays of 100-400 hits and 3D rays of ~60
 // hits keep 8 lanes busy
@@ -52,6 +53,16 @@ constexpr int RAY1_BLOCK = 128;               // rays (threads) per block of k_r
 // 26.0 / 15.8; on 128^2 rings of 2048, 8192, 10368 and 18432: 5.9 / 6.5,
 // 6.3 / 6.4, 6.9 / 6.4 and 7.4 / 6.6
 constexpr long long RAY1_MIN_RAYS = 10240;
+// the same in 3D, where the lanes form reads the volume itself and the thread
+// form's copy costs a launch and the volume twice: its latency while the copy
+// does not fill the GPU, then its bytes.  Rays at which both take the same time
+// (us there), by the cube's side: 16 40 - 80K (the launches' latency, which differs
+// between machines), 24 and 32 54K (5.1, 5.9), 48 75K (8), 64 105K (12), 80 126K (16), 100 150K (22), 112 190K (28), 128 235K (38); at a
+// tenth of them the copy alone makes it up to twice the time (100^3, 12800 rays:
+// 6.4 / 13.8)
+inline long long ray1_min_rays_3d(long long voxels) {
+	return 56 * 1024 + std::min(voxels / 5, 40LL * 1024) + voxels / 14;
+}
 
 struct OpBatch {
 	// dense (2d/mat_mult.h:15-36): forward gemv by rows; adjoint over

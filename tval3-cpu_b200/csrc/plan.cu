@@ -359,7 +359,10 @@ void prepare_op(cudaStream_t s, const tval3g_problem &p, int flags, OpStore &st,
 		d.scale = p.scale_factor;
 		d.rays = drays;
 		d.rays_fwd = drays;
-		const bool copies = is3 && nr >= RAY1_MIN_RAYS && !(flags & PLAN_LEAN);   // for the thread-per-ray form
+		// for the thread-per-ray form: where a launch of these rays takes it, or one
+		// of a batch may
+		const bool copies = is3 && !(flags & PLAN_LEAN) &&
+		                    nr >= (flags & PLAN_BATCH ? RAY1_MIN_RAYS : ray1_min_rays_3d((long long)p.rv_x * p.rv_y * p.rv_z));
 		if (copies) {
 			int4 *sorted = sort_rays_3d(s, (int)nr, drays, (long long)nmp * E);
 			st.owned.push_back(sorted);
@@ -606,17 +609,21 @@ static long long build_op_maps(std::vector<Inst> &inst, const std::vector<OpStor
 	}
 	// ray forwards by lanes per ray: unless tuned, one thread per ray where the
 	// launch has enough of them, else RAY_SUBW lanes (the same sums)
-	long long rays[2] = {0, 0};
+	long long rays[2] = {0, 0}, voxels = 0;
 	for (int i = 0; i < cnt; i++) {
 		const OpDev &d = inst[i].op;
-		if (d.xT && d.fwd_lanes == 0) rays[d.kind == TVAL3G_OP_RAY3D] += d.nrays;
+		if (!d.xT || d.fwd_lanes != 0) continue;
+		const bool is3 = d.kind == TVAL3G_OP_RAY3D;
+		rays[is3] += d.nrays;
+		if (is3) voxels += (long long)d.rvx * d.rvy * d.tslices;
 	}
+	const bool threads[2] = {rays[0] >= RAY1_MIN_RAYS, rays[1] >= ray1_min_rays_3d(voxels)};
 	for (int dim3 = 0; dim3 < 2; dim3++)
 		for (int c = 0; c < 4; c++) {
 			for (int i = 0; i < cnt; i++) {
 				const OpDev &d = inst[i].op;
 				if (d.kind != (dim3 ? TVAL3G_OP_RAY3D : TVAL3G_OP_RAY2D)) continue;
-				const int lanes = d.fwd_lanes > 0 ? d.fwd_lanes : (d.xT && rays[dim3] >= RAY1_MIN_RAYS) ? 1 : RAY_SUBW;
+				const int lanes = d.fwd_lanes > 0 ? d.fwd_lanes : (d.xT && threads[dim3]) ? 1 : RAY_SUBW;
 				if (lanes != RAY_LANES[c]) continue;
 				const int rpb = lanes == 1 ? RAY1_BLOCK : 256 / lanes;
 				tb.add(i, (d.nrays + rpb - 1) / rpb);
@@ -627,7 +634,7 @@ static long long build_op_maps(std::vector<Inst> &inst, const std::vector<OpStor
 		for (int i = 0; i < cnt; i++) {
 			const OpDev &d = inst[i].op;
 			if (d.kind != (dim3 ? TVAL3G_OP_RAY3D : TVAL3G_OP_RAY2D) || !d.xT) continue;
-			if (dim3 && (d.fwd_lanes > 0 || rays[1] < RAY1_MIN_RAYS)) continue;   // only the thread form reads it
+			if (dim3 && (d.fwd_lanes > 0 || !threads[1])) continue;   // only the thread form reads it
 			tb.add(i, (long long)((d.rvx + 31) / 32) * ((d.tH + 31) / 32) * d.tslices);
 		}
 		tb.close(dim3 ? &ob.ray3_transpose : &ob.ray2_transpose);
@@ -745,7 +752,7 @@ Plan::Plan(int count, const tval3g_problem *probs, const tval3g_options *opts, i
 			                  : (p.op_kind == TVAL3G_OP_RAY3D) ? (long long)p.numPaths * p.numMPs
 			                  : (long long)p.m * (p.dims == 3 ? 1 : p.layers);
 			long long n = validate(p, b_len, 0, false);   // the callers validated p
-			prepare_op(stream_, p, flags | (lean ? PLAN_LEAN : 0), ops_[i], false);
+			prepare_op(stream_, p, flags | (lean ? PLAN_LEAN : 0) | (count > 1 ? PLAN_BATCH : 0), ops_[i], false);
 			Inst &I = h_inst_[i];
 			const int planes = p.complex_data ? 2 : 1;   // complex: real and imaginary planes
 			I.dims = p.dims; I.p = p.dim_y; I.q = p.dim_x; I.r = p.dims == 3 ? p.dim_z : planes;

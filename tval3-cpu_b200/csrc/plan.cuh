@@ -48,6 +48,8 @@ long long build_op_maps_upload(std::vector<Inst> &inst, const std::vector<OpStor
 constexpr int PLAN_SCHEDULE = 1 << 16;
 // internal flag of prepare_op: without the copies that only make a 3D forward faster
 constexpr int PLAN_LEAN = 1 << 17;
+// internal flag of prepare_op: more operators share its launches
+constexpr int PLAN_BATCH = 1 << 18;
 
 class Plan {
 public:

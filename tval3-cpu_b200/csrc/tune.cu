@@ -5,7 +5,7 @@
 // on-the-fly Bresenham forward (4, 8, 16 or one thread) and the sub-warp width of the
 // compressed gathers (4, 8, 16 or 32 lanes per CSR row, CSC column or 3D
 // pixel list).  Without tuning they follow built-in rules (one thread
-// per ray from RAY1_MIN_RAYS rays a launch, else 8 lanes; width by mean line
+// per ray from RAY1_MIN_RAYS (3D: ray1_min_rays_3d) rays a launch, else 8 lanes; width by mean line
 // length).  With TVAL3G_TUNE an operator is timed under
 // every candidate on its own data once, right after it is built, and keeps
 // the fastest; the choice is cached per operator signature (kind, sizes,
@@ -88,7 +88,7 @@ std::string device_tag() {
 std::string signature(const OpStore &st, long long rows, long long cols) {
 	const OpDev &d = st.dev;
 	std::ostringstream k;
-	k << "v2 kind=" << d.kind << " rows=" << rows << " cols=" << cols << " layers=" << d.layers
+	k << "v3 kind=" << d.kind << " rows=" << rows << " cols=" << cols << " layers=" << d.layers
 	  << " nnz=" << st.nnz << " rays=" << d.nrays << " tiled=" << d.tiled << " " << device_tag();
 	std::string s = k.str();
 	for (char &ch : s)
